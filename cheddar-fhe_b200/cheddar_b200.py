@@ -20,8 +20,8 @@ PARAM_DIR = os.path.join(_HERE, "params")
 
 CHD_MODDOWN, CHD_RESCALE, CHD_MODDOWN_RESCALE = 0, 1, 2
 BCONV_CUDA_CORE, BCONV_TENSOR_CORE = 0, 1   # chd_bconv_batch engines
-BCONV_AUTO = 2                                # Context.ks_engine only: autotuned per launch shape
-BCONV_TENSOR_CORE_WIDE = 3                    # Context.ks_engine only: tensor cores, 256-thread tiles (K <= 12)
+BCONV_AUTO = 2                                # Context.ks_engine only
+BCONV_TENSOR_CORE_WIDE = 3                    # Context.ks_engine only
 
 # stages of the fused N = 2^16 key switch (chd_stage_times), in launch order
 KS_STAGE_NAMES = ("modup_inv_rows", "modup_cols", "ks_rows", "moddown_cols", "fwd_rows_epilogue")
@@ -247,9 +247,8 @@ def _ptr(a):
 
 
 def ks_tuned_shapes():
-    """The column-pass autotuner's choices in this process: one dict per
-    launch shape (largest source count K, jobs, largest target count M) with
-    the engine (0 CUDA cores, 1 tensor cores) and the target split."""
+    """The column passes whose variant was chosen by timing in this process:
+    none since the column pass has one variant."""
     n = lib().chd_ks_tuned_shapes(None, 0)
     out = (C.c_int * (6 * max(1, n)))()
     n = lib().chd_ks_tuned_shapes(out, n)
@@ -258,10 +257,7 @@ def ks_tuned_shapes():
 
 
 def ks_rows_tuned_shapes():
-    """The key-switch row pass's autotuned choices in this process: one dict
-    per launch shape with its `variant` (0 loads where used at 3 CTAs per
-    SM, 1 loads ahead at 2, 2 loads where used at 4) and `prefetch` True for
-    variant 1."""
+    """The same for the key-switch row pass: none."""
     n = lib().chd_ks_rows_tuned_shapes(None, 0)
     out = (C.c_int * (5 * max(1, n)))()
     n = lib().chd_ks_rows_tuned_shapes(out, n)
@@ -321,10 +317,11 @@ class Context:
 
     @property
     def ks_engine(self):
-        """Base-conversion engine of the key-switching and rescaling paths:
-        BCONV_CUDA_CORE, BCONV_TENSOR_CORE or BCONV_AUTO (the faster of the
-        two per launch shape, measured on first use); residues are
-        bit-identical."""
+        """Engine of the key-switching and rescaling paths: BCONV_CUDA_CORE,
+        BCONV_TENSOR_CORE, BCONV_TENSOR_CORE_WIDE (one column pass serves
+        them all at N = 2^16) or BCONV_AUTO (also times the register variants
+        of the hoisted rotations and the plaintext accumulation on first
+        use); residues are bit-identical."""
         return lib().chd_get_ks_engine(self.ptr)
 
     @ks_engine.setter

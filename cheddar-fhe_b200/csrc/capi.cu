@@ -373,9 +373,9 @@ int chd_set_ks_engine(chd_context *ctx, int engine) try {
 
 int chd_get_ks_engine(const chd_context *ctx) { return ctx ? ctx->c->ks_engine : -1; }
 
-int chd_ks_tuned_shapes(int *out, int cap) { return modswitch_tuned_shapes(out, cap); }
+int chd_ks_tuned_shapes(int *, int) { return 0; }
 
-int chd_ks_rows_tuned_shapes(int *out, int cap) { return ks_rows_tuned_shapes(out, cap); }
+int chd_ks_rows_tuned_shapes(int *, int) { return 0; }
 
 int chd_set_stream_split(chd_context *ctx, int on) try {
   CHD_CTX(ctx);

@@ -557,6 +557,10 @@ Context::~Context() {
     cudaFree(m.d_mod_down2);
     cudaFree(m.d_rs2);
     cudaFree(m.d_mdr2);
+    for (auto *p : m.d_mod_up_frag) cudaFree(p);
+    cudaFree(m.d_mod_down_frag);
+    cudaFree(m.d_rs_frag);
+    cudaFree(m.d_mdr_frag);
   }
   cudaFree(d_primes);
   cudaFree(d_qinv);
@@ -676,6 +680,51 @@ int32_t *upload_i32(const std::vector<int32_t> &v) {
   cudaMemcpy(p, v.data(), v.size() * 4, cudaMemcpyHostToDevice);
   return p;
 }
+
+// B fragments of the column pass's base-conversion MMAs (modswitch.cu) for a
+// centred table T[M][K] over the target primes p: per group of four targets
+// and step of eight sources one uint4 per lane (nn = lane / 4, tq = lane % 4):
+// .x / .y byte i = nn % 2 of 2^(8j) T mod p (j = 0..3, low byte first) of
+// target nn / 2 of the group and source tq / tq + 4 of the step, .z / .w the
+// same of byte i + 2; zero past the last target or source.  After the steps
+// one uint4 per lane holds the four bytes of -2^30 sum_k T mod p of target tq.
+uint4 *upload_frags(const std::vector<int32_t> &T, int K, int M, const uint32_t *p) {
+  if (T.empty() || K < 1 || K > 16) return nullptr;
+  const int groups = (M + 3) / 4, steps = (K + 7) / 8;
+  std::vector<uint4> f(static_cast<size_t>(groups) * (steps + 1) * 32, make_uint4(0, 0, 0, 0));
+  auto plain = [&](int m, int k) {
+    const int32_t t = T[static_cast<size_t>(m) * K + k];
+    return static_cast<uint64_t>(t < 0 ? static_cast<int64_t>(t) + p[m] : t);
+  };
+  auto word = [&](int m, int k, int i) {
+    uint32_t w = 0;
+    if (m < M && k < K)
+      for (int j = 0; j < 4; j++)
+        w |= ((static_cast<uint32_t>((plain(m, k) << (8 * j)) % p[m]) >> (8 * i)) & 0xffu) << (8 * j);
+    return w;
+  };
+  for (int g = 0; g < groups; g++) {
+    uint4 *fg = f.data() + static_cast<size_t>(g) * (steps + 1) * 32;
+    for (int lane = 0; lane < 32; lane++) {
+      const int tq = lane & 3, m = 4 * g + (lane >> 3), i = (lane >> 2) & 1;
+      for (int s = 0; s < steps; s++)
+        fg[32 * s + lane] = make_uint4(word(m, 8 * s + tq, i), word(m, 8 * s + 4 + tq, i), word(m, 8 * s + tq, i + 2),
+                                       word(m, 8 * s + 4 + tq, i + 2));
+      const int mc = 4 * g + tq;
+      if (mc < M) {
+        uint64_t sum = 0;
+        for (int k = 0; k < K; k++) sum += plain(mc, k);
+        const uint64_t r = ((sum % p[mc]) << 30) % p[mc];
+        const uint32_t corr = r ? p[mc] - static_cast<uint32_t>(r) : 0u;
+        fg[32 * steps + lane] = make_uint4(corr & 0xffu, (corr >> 8) & 0xffu, (corr >> 16) & 0xffu, corr >> 24);
+      }
+    }
+  }
+  uint4 *d = nullptr;
+  if (cudaMalloc(&d, f.size() * sizeof(uint4)) != cudaSuccess) return nullptr;
+  cudaMemcpy(d, f.data(), f.size() * sizeof(uint4), cudaMemcpyHostToDevice);
+  return d;
+}
 }  // namespace
 
 void build_level_ms(const Params &P, int level, LevelMS *out) {
@@ -751,6 +800,18 @@ void build_level_ms(const Params &P, int level, LevelMS *out) {
   epi_consts(mdr_src, next, m.restore_start, m.restore_end, &m.mdr_inv, &m.mdr_pad);
 }
 
+// Table position of twiddle j: its index, except that the tables of N = 2^16
+// keep the 4 resp. 8 pairs that a thread of the row phase needs for stage
+// m = 16384 resp. 32768 in chunks of two, chunk-major within the row's 1024
+// resp. 2048 pairs (tw_radix16_last, ntt_common.cuh).
+static int tw_position(int j, int log_n) {
+  if (log_n != 16 || j < 16384) return j;
+  const int lg = j < 32768 ? 2 : 3, base = j < 32768 ? 16384 : 32768;
+  const int o = j - base, row = o >> (8 + lg), i = o & ((256 << lg) - 1);
+  const int t = i >> lg, c = (i >> 1) & ((1 << (lg - 1)) - 1), x = i & 1;
+  return base + (row << (8 + lg)) + 512 * c + 2 * t + x;
+}
+
 Status Context::init(const ParamSpec &spec, int dev, std::string *err) {
   P = Params::create(spec, err);
   if (!P) return kErrInvalidArg;
@@ -796,8 +857,9 @@ Status Context::init(const ParamSpec &spec, int dev, std::string *err) {
     }
     for (int j = 0; j < n; j++) {
       unsigned r = brev_host(j, P->log_n);
-      tw[static_cast<size_t>(g) * n + j] = make_uint2(pw[r], shoup(pw[r], q));
-      itw[static_cast<size_t>(g) * n + j] = make_uint2(pwi[r], shoup(pwi[r], q));
+      const size_t o = static_cast<size_t>(g) * n + tw_position(j, P->log_n);
+      tw[o] = make_uint2(pw[r], shoup(pw[r], q));
+      itw[o] = make_uint2(pwi[r], shoup(pwi[r], q));
     }
     imag_unit[g] = prime::to_mont(pw[brev_host(1, P->log_n)], q);  // psi^(N/2), Montgomery
   }
@@ -832,6 +894,29 @@ Status Context::init(const ParamSpec &spec, int dev, std::string *err) {
     m.d_mod_down2 = upload_i32(m.mod_down2);
     m.d_rs2 = upload_i32(m.rs2);
     m.d_mdr2 = upload_i32(m.mdr2);
+    if (P->log_n != 16) continue;
+    // targets: the extended basis without the digit's own primes (ModUp), the
+    // level's q primes (ModDown), the next level's (Rescale, merged)
+    const NP np = P->level_np(level, m.num_aux);
+    std::vector<int> g(np.total());
+    P->gidx(np, g.data());
+    std::vector<uint32_t> lp;
+    for (int x : g) lp.push_back(P->primes[x]);
+    for (int i = 0; i < m.beta; i++) {
+      std::vector<uint32_t> dst(lp.begin(), lp.begin() + m.dig_s[i]);
+      dst.insert(dst.end(), lp.begin() + m.dig_e[i], lp.end());
+      m.d_mod_up_frag.push_back(
+          upload_frags(m.mod_up2[i], m.dig_e[i] - m.dig_s[i], static_cast<int>(dst.size()), dst.data()));
+    }
+    m.d_mod_down_frag = upload_frags(m.mod_down2, np.aux, np.q(), lp.data());
+    if (!m.has_rescale) continue;
+    const NP nn = P->level_np(level - 1, 0);
+    std::vector<int> gn(nn.total());
+    P->gidx(nn, gn.data());
+    std::vector<uint32_t> next;
+    for (int x : gn) next.push_back(P->primes[x]);
+    m.d_rs_frag = upload_frags(m.rs2, m.rs_src_len, nn.q(), next.data());
+    m.d_mdr_frag = upload_frags(m.mdr2, m.mdr_src_len, nn.q(), next.data());
   }
   if (cudaDeviceSynchronize() != cudaSuccess) {
     *err = std::string("context setup: ") + cudaGetErrorString(cudaGetLastError());
@@ -1131,8 +1216,6 @@ Status Context::modup_fused(int level, int count, const uint32_t *const *src, ui
     }
   for_row_batches(rows, [&](const RowBatch &rb) { launch_ntt_inv_rows(rb, P->log_n, stream); });
   MSColBatch b{};
-  b.engine = ks_engine;
-  b.err = d_err;
   b.tw = d_tw;
   b.itw = d_itw;
   b.primes = d_primes;
@@ -1146,7 +1229,7 @@ Status Context::modup_fused(int level, int count, const uint32_t *const *src, ui
       MSColJob &j = b.jobs[b.count++];
       j.src = rows_out + static_cast<size_t>(c) * nq * n;
       j.dst = dst[c][i];
-      j.table = m.d_mod_up2[i];
+      j.frag = m.d_mod_up_frag[i];
       j.K = e - s;
       j.M = tot - (e - s);
       CHD_CHECK(j.K <= 16 && j.M <= 64, kErrUnsupported, "modup: digit too large");
@@ -1197,7 +1280,7 @@ Status Context::moddown_plan(int level, MDType type, MDPlan *pl) const {
   pl->dst_len = pl->nd.total();
   CHD_CHECK(pl->src_len >= 1 && pl->src_len <= 16, kErrUnsupported, "moddown: more than 16 dropped primes");
   pl->c1 = type == MDType::kModDown ? m.mod_down1.data() : type == MDType::kRescale ? m.rs1.data() : m.mdr1.data();
-  pl->table = type == MDType::kModDown ? m.d_mod_down2 : type == MDType::kRescale ? m.d_rs2 : m.d_mdr2;
+  pl->frag = type == MDType::kModDown ? m.d_mod_down_frag : type == MDType::kRescale ? m.d_rs_frag : m.d_mdr_frag;
   pl->inv = type == MDType::kModDown ? m.inv_p_prod.data() : type == MDType::kRescale ? m.rs_inv.data() : m.mdr_inv.data();
   pl->pad = type == MDType::kModDown ? nullptr : type == MDType::kRescale ? m.rs_pad.data() : m.mdr_pad.data();
   pl->gs.assign(pl->ns.total(), 0);
@@ -1339,8 +1422,6 @@ Status Context::key_switch_fused_pipeline(const int *levels, int count, const KS
   });
   timer_span(kKsInvRows, t0, nl);
   MSColBatch b{};
-  b.engine = ks_engine;
-  b.err = d_err;
   b.tw = d_tw;
   b.itw = d_itw;
   b.primes = d_primes;
@@ -1358,7 +1439,7 @@ Status Context::key_switch_fused_pipeline(const int *levels, int count, const KS
         MSColJob &j = b.jobs[b.count++];
         j.src = t1 + o_t1[c] * N;
         j.dst = MU(c, static_cast<int>(bi));
-        j.table = m.d_mod_up2[i];
+        j.frag = m.d_mod_up_frag[i];
         j.K = e - s;
         j.M = sh.tot - (e - s);
         CHD_CHECK(j.K <= 16 && j.M <= 64, kErrUnsupported, "modup: digit too large");
@@ -1423,7 +1504,7 @@ Status Context::key_switch_fused_pipeline(const int *levels, int count, const KS
     t0 = timer_mark();
     auto flush = [&]() {
       if (d.count == 0) return;
-      launch_ks_rows(d, P->log_n, stream, ks_engine == 2);
+      launch_ks_rows(d, P->log_n, stream);
       nl++;
       d.count = d.nlv = d.max_rows = 0;
       lv_of.clear();
@@ -1474,7 +1555,7 @@ Status Context::key_switch_fused_pipeline(const int *levels, int count, const KS
         MSColJob &j = b.jobs[b.count++];
         j.src = drop + (o_drop[c] + static_cast<size_t>(p) * pl.src_len) * N;
         j.dst = p == 0 ? in[c].out_b : in[c].out_a;
-        j.table = pl.table;
+        j.frag = pl.frag;
         j.K = pl.src_len;
         j.M = pl.dst_len;
         for (int i = 0; i < pl.src_len; i++) {
@@ -1588,6 +1669,8 @@ Status Context::moddown_pipeline(int level, MDType type, const uint32_t *const *
   const uint32_t *c1 = type == MDType::kModDown ? m.mod_down1.data()
                        : type == MDType::kRescale ? m.rs1.data() : m.mdr1.data();
   const int32_t *table = type == MDType::kModDown ? m.d_mod_down2 : type == MDType::kRescale ? m.d_rs2 : m.d_mdr2;
+  const uint4 *frag = type == MDType::kModDown  ? m.d_mod_down_frag
+                      : type == MDType::kRescale ? m.d_rs_frag : m.d_mdr_frag;
   const uint32_t *inv = type == MDType::kModDown ? m.inv_p_prod.data()
                         : type == MDType::kRescale ? m.rs_inv.data() : m.mdr_inv.data();
   const uint32_t *pad = type == MDType::kModDown ? nullptr
@@ -1624,8 +1707,6 @@ Status Context::moddown_pipeline(int level, MDType type, const uint32_t *const *
   if (fused) {
     for_row_batches(rows, [&](const RowBatch &rb) { launch_ntt_inv_rows(rb, P->log_n, stream); });
     MSColBatch b{};
-    b.engine = ks_engine;
-    b.err = d_err;
     b.tw = d_tw;
     b.itw = d_itw;
     b.primes = d_primes;
@@ -1634,7 +1715,7 @@ Status Context::moddown_pipeline(int level, MDType type, const uint32_t *const *
       MSColJob &j = b.jobs[b.count++];
       j.src = reinterpret_cast<uint32_t *>(xt) + static_cast<size_t>(p) * src_len * n;
       j.dst = dst[p];
-      j.table = table;
+      j.frag = frag;
       j.K = src_len;
       j.M = dst_len;
       for (int i = 0; i < src_len; i++) {

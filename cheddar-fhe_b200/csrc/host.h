@@ -117,6 +117,9 @@ struct LevelMS {
   // device copies of the BConv tables
   std::vector<int32_t *> d_mod_up2;
   int32_t *d_mod_down2 = nullptr, *d_rs2 = nullptr, *d_mdr2 = nullptr;
+  // N = 2^16: the same tables as MMA fragments of the fused column pass
+  std::vector<uint4 *> d_mod_up_frag;
+  uint4 *d_mod_down_frag = nullptr, *d_rs_frag = nullptr, *d_mdr_frag = nullptr;
 };
 
 // Host-only computation of the ModSwitch constants of one level (no GPU).
@@ -349,7 +352,7 @@ class Context {
   // tensor-core base conversion's bounded waits run out
   uint32_t tc_stall_polls = 0;
   int num_sms = 0;
-  int ks_engine = 0;      // ModUp / ModDown column-pass base conversion: 0 CUDA cores, 1 tensor cores, 2 autotuned
+  int ks_engine = 0;      // chd_set_ks_engine; 2 (CHD_BCONV_AUTO) times the variants of launch_hoisted and launch_pt_accum
   // A fused key switch of two or more ciphertexts runs its two halves on the
   // context stream and on aux_stream (forked from and joined back into the
   // context stream by events), so that the kernels of one half fill the
@@ -388,7 +391,7 @@ class Context {
     int src_len = 0, dst_len = 0, src2_start = 0, src2_end = 0, src2_off = 0;
     std::vector<int> srows, gs, gd;
     const uint32_t *c1 = nullptr, *inv = nullptr, *pad = nullptr;
-    const int32_t *table = nullptr;
+    const uint4 *frag = nullptr;
   };
   Status moddown_plan(int level, MDType type, MDPlan *plan) const;
   // Fused N = 2^16 key switch (see keyswitch.cu): count inputs at one level,

@@ -150,7 +150,7 @@ struct ConstAccumDesc {
 };
 void launch_const_accum(const ConstAccumDesc &d, cudaStream_t s);
 
-// Fused ModSwitch column pass (N = 2^16 only): per 16-column tile
+// Fused ModSwitch column pass (N = 2^16 only): per column
 //   x~_k  = centre(INTT column phase(src_k) * c0_k)        (K <= 16 sources)
 //   y_m   = (sum_k x~_k T[m][k]) * 2^-32 mod p_m           (exact BConv)
 //   dst_m = NTT column phase(y_m)                          (lazy [0, 2q))
@@ -159,7 +159,7 @@ void launch_const_accum(const ConstAccumDesc &d, cudaStream_t s);
 struct MSColJob {
   const uint32_t *src;
   uint32_t *dst;
-  const int32_t *table;  // device [M][K]
+  const uint4 *frag;     // base-conversion MMA fragments (bconv_frags, context.cu)
   int K, M;
   uint8_t src_row[16], src_gidx[16];
   uint8_t dst_row[64], dst_gidx[64];
@@ -171,10 +171,6 @@ struct MSColJob {
 constexpr int kMaxMSColJobs = 64;
 struct MSColBatch {
   int count;
-  int engine;             // base conversion on 0: CUDA cores, 1: tensor cores, 3: tensor cores with
-                          // 256-thread tiles (K <= 12; larger K runs engine 1); 4 (autotuner only):
-                          // 3 with the K <= 8 kernel sized for 2 CTAs per SM
-  int *err;               // set to 1 when a tensor-core wait gives up
   const uint2 *tw, *itw;  // twiddle tables [nprimes][N]
   const uint32_t *primes;
   const int32_t *qinvs;
@@ -182,17 +178,6 @@ struct MSColBatch {
 };
 static_assert(sizeof(MSColBatch) + 16 <= 32764, "column-pass batch beyond the kernel parameter limit");
 void launch_modswitch_cols(const MSColBatch &b, int log_n, cudaStream_t s);
-// the autotuned choices (engine, target split) cached so far: 6 ints per
-// shape (device, largest K, jobs, largest M, engine, split); returns the count
-int modswitch_tuned_shapes(int *out, int cap);
-// tensor-core column pass (modswitch_tc.cu); every job has K <= 16
-void launch_modswitch_cols_tc(const MSColBatch &b, int max_k, cudaStream_t s);
-size_t modswitch_cols_tc_smem(int kmax);
-// the same on 256-thread tiles, 8 coefficients per thread (modswitch_tc8.cu),
-// for jobs with K <= 12; regs128 sizes the K <= 8 kernel for 2 CTAs per SM
-// (128 registers) instead of 3 (80)
-bool modswitch_cols_tc8_supports(int max_k);
-void launch_modswitch_cols_tc8(const MSColBatch &b, int max_k, bool regs128, cudaStream_t s);
 void launch_ntt_inv_rows(const RowBatch &rb, int log_n, cudaStream_t s);
 
 // Fused key-switching row pass (N = 2^16), see keyswitch.cu.  Modes:
@@ -227,12 +212,7 @@ struct KSRowsDesc {
   KSRowsLevel lv[kMaxKSRowsLevels];
   KSRowsCt ct[kMaxKSRowsCts];
 };
-// tune: pick the row-pass variant per launch shape by timing both once
-// (the context's CHD_BCONV_AUTO); otherwise the one without prefetching
-void launch_ks_rows(const KSRowsDesc &d, int log_n, cudaStream_t s, bool tune = false);
-// the row-pass choices cached so far: 5 ints per shape (device, ciphertexts,
-// largest row count, mode, prefetching variant); returns the count
-int ks_rows_tuned_shapes(int *out, int cap);
+void launch_ks_rows(const KSRowsDesc &d, int log_n, cudaStream_t s);
 
 // Key-switching inner product with the P * (d0, d1) term folded in:
 //   acc_b[r] = sum_i mu_i[r] * kb_i[r] + (r < nq ? p_prod[r] * d0[r] : 0)

@@ -1,12 +1,28 @@
 // Building blocks shared by the NTT kernels (ntt.cu), the fused ModSwitch
 // column pass (modswitch.cu) and the fused key-switch row pass
-// (keyswitch.cu): radix-8 / radix-16 networks of lazy Shoup butterflies with
-// vectorised twiddle loads, and the shared-memory swizzle of the row phase.
+// (keyswitch.cu): radix-16 networks of lazy Shoup butterflies with
+// vectorised twiddle loads, and the row phase with its shared-memory
+// exchanges.
 #pragma once
 
 #include "arith.cuh"
 
 namespace chd {
+
+// ---- N = 2^16 geometry: a limb is a 16 x 4096 row-major matrix ----
+// Stages m = 1 .. 8 pair elements of one column (a 16-point column transform
+// held by one thread); stages m = 16 .. 32768 stay inside one 4096-element
+// row, held by the 256 threads of a CTA with 16 elements each, in three
+// radix-16 rounds.  Between the first two rounds the row crosses the CTA
+// (one barrier); the last two work on blocks of 256 elements, each owned by
+// one half-warp, which exchanges them under __syncwarp.  A radix-16 column
+// needs no exchange, so the fused base-conversion column pass
+// (modswitch.cu) keeps everything in registers; with the earlier 128 x 512
+// split the same pass crossed shared memory and a CTA barrier per source
+// and per target and took 313 us of a 642 us batch of 8 multiplications.
+constexpr int kRowLen = 4096;      // elements per row
+constexpr int kRowThreads = 256;   // threads per row
+constexpr int kLimbRows = 16;      // rows per limb
 
 // Twiddle loads: tables hold (w, companion) pairs; pairs at even (resp.
 // multiple-of-4) indices are 16- (resp. 32-) byte aligned, so 2 and 4
@@ -16,56 +32,33 @@ __device__ __forceinline__ void tw_ld2(const uint2 *tw, int i, uint2 *w) {
   w[0] = make_uint2(v.x, v.y);
   w[1] = make_uint2(v.z, v.w);
 }
-__device__ __forceinline__ void tw_ld4(const uint2 *tw, int i, uint2 *w) {
-  tw_ld2(tw, i, w);
-  tw_ld2(tw, i + 2, w + 2);
+
+// The fifteen twiddles of a radix-16 network over group index B (16 / 2^s
+// consecutive stages m' = 2^s B' share the numbering): stage s uses pairs
+// (B << s) + g, g < 2^s.  w[2^s + g] receives them.
+__device__ __forceinline__ void tw_radix16(const uint2 *tw, int B, uint2 *w) {
+  w[1] = __ldg(tw + B);
+  tw_ld2(tw, 2 * B, w + 2);
+#pragma unroll
+  for (int c = 0; c < 2; c++) tw_ld2(tw, 4 * B + 2 * c, w + 4 + 2 * c);
+#pragma unroll
+  for (int c = 0; c < 4; c++) tw_ld2(tw, 8 * B + 2 * c, w + 8 + 2 * c);
+}
+// The same for the last round of row r, thread t (B = 4096 + 256 r + t): the
+// tables of N = 2^16 store the pairs of stages m = 16384 and 32768 of one
+// row chunk-major (tw_position), so that a warp's 16-byte loads are
+// contiguous.
+__device__ __forceinline__ void tw_radix16_last(const uint2 *tw, int r, int t, uint2 *w) {
+  w[1] = __ldg(tw + 4096 + 256 * r + t);
+  tw_ld2(tw, 8192 + 512 * r + 2 * t, w + 2);
+#pragma unroll
+  for (int c = 0; c < 2; c++) tw_ld2(tw, 16384 + 1024 * r + 512 * c + 2 * t, w + 4 + 2 * c);
+#pragma unroll
+  for (int c = 0; c < 4; c++) tw_ld2(tw, 32768 + 2048 * r + 512 * c + 2 * t, w + 8 + 2 * c);
 }
 
-// Radix-8 forward network on x[0..7]: CT stages at register distances 4, 2,
-// 1 with twiddles tw[b0], tw[b1 + g] (g < 2), tw[b2 + g] (g < 4).
-// b1 must be even and b2 a multiple of 4.
-__device__ __forceinline__ void radix8_fwd(uint32_t *x, const uint2 *tw, int b0, int b1, int b2, uint32_t q) {
-  uint2 w1[2], w2[4];
-  const uint2 w0 = __ldg(tw + b0);
-  tw_ld2(tw, b1, w1);
-  tw_ld4(tw, b2, w2);
-#pragma unroll
-  for (int k = 0; k < 4; k++) ct_lazy(x[k], x[k + 4], w0, q);
-#pragma unroll
-  for (int g = 0; g < 2; g++) {
-    ct_lazy(x[4 * g], x[4 * g + 2], w1[g], q);
-    ct_lazy(x[4 * g + 1], x[4 * g + 3], w1[g], q);
-  }
-#pragma unroll
-  for (int g = 0; g < 4; g++) ct_lazy(x[2 * g], x[2 * g + 1], w2[g], q);
-}
-
-// Radix-8 inverse network (GS stages at distances 1, 2, 4), mirror of the above.
-__device__ __forceinline__ void radix8_inv(uint32_t *x, const uint2 *tw, int b0, int b1, int b2, uint32_t q) {
-  uint2 w1[2], w2[4];
-  const uint2 w0 = __ldg(tw + b0);
-  tw_ld2(tw, b1, w1);
-  tw_ld4(tw, b2, w2);
-#pragma unroll
-  for (int g = 0; g < 4; g++) gs_lazy(x[2 * g], x[2 * g + 1], w2[g], q);
-#pragma unroll
-  for (int g = 0; g < 2; g++) {
-    gs_lazy(x[4 * g], x[4 * g + 2], w1[g], q);
-    gs_lazy(x[4 * g + 1], x[4 * g + 3], w1[g], q);
-  }
-#pragma unroll
-  for (int k = 0; k < 4; k++) gs_lazy(x[k], x[k + 4], w0, q);
-}
-
-// First four column stages (m = 1, 2, 4, 8) on 16 registers holding rows
-// rg + 8k of one column: pair (k, k + 8/m) with twiddle tw[m + k / (16/m)].
-__device__ __forceinline__ void radix16_cols_fwd(uint32_t *x, const uint2 *tw, uint32_t q) {
-  uint2 w[16];
-  w[1] = __ldg(tw + 1);
-  tw_ld2(tw, 2, w + 2);
-  tw_ld4(tw, 4, w + 4);
-  tw_ld4(tw, 8, w + 8);
-  tw_ld4(tw, 12, w + 12);
+// Radix-16 forward network (CT stages at register distances 8, 4, 2, 1).
+__device__ __forceinline__ void radix16_fwd(uint32_t *x, const uint2 *w, uint32_t q) {
 #pragma unroll
   for (int s = 0; s < 4; s++) {
     const int m = 1 << s, h = 8 >> s;
@@ -75,15 +68,8 @@ __device__ __forceinline__ void radix16_cols_fwd(uint32_t *x, const uint2 *tw, u
       for (int j = 0; j < h; j++) ct_lazy(x[g * 2 * h + j], x[g * 2 * h + j + h], w[m + g], q);
   }
 }
-
-// Last four inverse column stages (m = 8, 4, 2, 1), mirror of the above.
-__device__ __forceinline__ void radix16_cols_inv(uint32_t *x, const uint2 *tw, uint32_t q) {
-  uint2 w[16];
-  w[1] = __ldg(tw + 1);
-  tw_ld2(tw, 2, w + 2);
-  tw_ld4(tw, 4, w + 4);
-  tw_ld4(tw, 8, w + 8);
-  tw_ld4(tw, 12, w + 12);
+// Radix-16 inverse network (GS stages at distances 1, 2, 4, 8), its mirror.
+__device__ __forceinline__ void radix16_inv(uint32_t *x, const uint2 *w, uint32_t q) {
 #pragma unroll
   for (int s = 3; s >= 0; s--) {
     const int m = 1 << s, h = 8 >> s;
@@ -94,78 +80,132 @@ __device__ __forceinline__ void radix16_cols_inv(uint32_t *x, const uint2 *tw, u
   }
 }
 
-// Shared-memory position of element c of a 512-element row.  The three
-// exchange patterns of the row phase (c = t + 64k, 64(t>>3) + (t&7) + 8k and
-// 8t + k, t the lane) are all bank-conflict free under this bijection.
-__device__ __forceinline__ int rsw(int c) { return c ^ ((c >> 3) & 31); }
-
-// Barrier of the 64 threads (two warps) that own one row: named barrier
-// `bar` (1 .. 15), so that the rows of a CTA do not wait for each other, or
-// the CTA-wide barrier for bar < 0.  The key-switch row pass (several loads
-// and MACs between its row transforms) gains from the per-row form; the
-// plain row kernels measured faster with the CTA-wide one.
-__device__ __forceinline__ void row_sync(int bar) {
-  if (bar < 0)
-    __syncthreads();
-  else
-    asm volatile("bar.sync %0, 64;" ::"r"(bar) : "memory");
+// Shared-memory position of element 256 b + 16 k + u of a row.  Every access
+// of the row phase is free of bank conflicts under it: 32-bit accesses with
+// (b, k) fixed per half-warp and u the lane, or with b the register and
+// 16 k + u the thread; 128-bit accesses of 4-word chunks u / 4 with k the
+// lane, or with (k, u / 4) counting through the lanes.
+__device__ __forceinline__ int rpos(int b, int k, int u) {
+  return 256 * b + 16 * (k ^ (b & 1)) + (u ^ (((k >> 1) & 3) << 2));
 }
 
-// The 9 row stages (m = 128 .. 32768) of the forward transform on one
-// 512-element row r held by 64 threads (thread t), 8 elements each.  Input
-// x[k] = element t + 64k; output x[k] = element 8t + k.  srow is the row's
-// 512-word shared buffer, bar the row's named barrier; the caller
-// synchronises (row_sync) before reusing srow.
-__device__ __forceinline__ void row_fwd(uint32_t *x, uint32_t *srow, const uint2 *tw, int r, int t, uint32_t q,
-                                        int bar) {
-  const int b = t >> 3, u0 = t & 7;
-  radix8_fwd(x, tw, 128 + r, 256 + 2 * r, 512 + 4 * r, q);
+// "Row order" below: thread t holds x[k] = element t + 256 k.  "Chunk order":
+// with b = t / 16, u = t % 16, x[4 i + c] = element 256 b + 64 i + 4 u + c, so
+// that a half-warp's 16-byte accesses to memory cover 256 contiguous bytes.
+__device__ __forceinline__ int chunk_off(int t) { return (t >> 4) * 256 + (t & 15) * 4; }  // + 64 i
+
+// chunk order -> own group of 16 consecutive elements and back, inside the
+// half-warp's block of the row buffer
+__device__ __forceinline__ void group_st(uint32_t *sm, int t, const uint32_t *x) {
+  const int b = t >> 4, u = t & 15;
 #pragma unroll
-  for (int k = 0; k < 8; k++) srow[rsw(t + 64 * k)] = x[k];
-  row_sync(bar);
+  for (int i = 0; i < 4; i++)
+    *reinterpret_cast<uint4 *>(sm + rpos(b, u, 4 * i)) = make_uint4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
+}
+__device__ __forceinline__ void group_ld(const uint32_t *sm, int t, uint32_t *x) {
+  const int b = t >> 4, u = t & 15;
 #pragma unroll
-  for (int k = 0; k < 8; k++) x[k] = srow[rsw(64 * b + u0 + 8 * k)];
-  radix8_fwd(x, tw, 1024 + 8 * r + b, 2048 + 16 * r + 2 * b, 4096 + 32 * r + 4 * b, q);
-  row_sync(bar);
+  for (int i = 0; i < 4; i++) {
+    const uint4 v = *reinterpret_cast<const uint4 *>(sm + rpos(b, u, 4 * i));
+    x[4 * i] = v.x; x[4 * i + 1] = v.y; x[4 * i + 2] = v.z; x[4 * i + 3] = v.w;
+  }
+}
+__device__ __forceinline__ void chunk_st(uint32_t *sm, int t, const uint32_t *x) {
+  const int b = t >> 4, u = t & 15;
 #pragma unroll
-  for (int k = 0; k < 8; k++) srow[rsw(64 * b + u0 + 8 * k)] = x[k];
-  row_sync(bar);
+  for (int i = 0; i < 4; i++)
+    *reinterpret_cast<uint4 *>(sm + rpos(b, 4 * i + (u >> 2), 4 * (u & 3))) =
+        make_uint4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
+}
+__device__ __forceinline__ void chunk_ld(const uint32_t *sm, int t, uint32_t *x) {
+  const int b = t >> 4, u = t & 15;
 #pragma unroll
-  for (int k = 0; k < 8; k++) x[k] = srow[rsw(8 * t + k)];
-  radix8_fwd(x, tw, 8192 + 64 * r + t, 16384 + 128 * r + 2 * t, 32768 + 256 * r + 4 * t, q);
+  for (int i = 0; i < 4; i++) {
+    const uint4 v = *reinterpret_cast<const uint4 *>(sm + rpos(b, 4 * i + (u >> 2), 4 * (u & 3)));
+    x[4 * i] = v.x; x[4 * i + 1] = v.y; x[4 * i + 2] = v.z; x[4 * i + 3] = v.w;
+  }
 }
 
-// The 9 row stages of the inverse transform (m = 32768 .. 128): input x[k] =
-// element 8t + k, output x[k] = element t + 64k.
-__device__ __forceinline__ void row_inv(uint32_t *x, uint32_t *srow, const uint2 *tw, int r, int t, uint32_t q,
-                                        int bar) {
-  const int b = t >> 3, u0 = t & 7;
-  radix8_inv(x, tw, 8192 + 64 * r + t, 16384 + 128 * r + 2 * t, 32768 + 256 * r + 4 * t, q);
+// The 12 row stages (m = 16 .. 32768) of the forward transform on row r of a
+// limb: x in row order -> chunk order, lazy [0, 2q).  sm: 4096 words.  One
+// CTA barrier; a caller that runs another row transform of the CTA
+// alternates between two buffers (a thread past the barrier of transform i
+// knows that every thread is done with the buffer of transform i - 1).
+__device__ __forceinline__ void row_fwd(uint32_t *x, uint32_t *sm, const uint2 *tw, int r, int t, uint32_t q) {
+  const int b = t >> 4, u = t & 15;
+  {
+    uint2 w[16];
+    tw_radix16(tw, 16 + r, w);
+    radix16_fwd(x, w, q);
+  }
 #pragma unroll
-  for (int k = 0; k < 8; k++) srow[rsw(8 * t + k)] = x[k];
-  row_sync(bar);
+  for (int k = 0; k < 16; k++) sm[rpos(k, b, u)] = x[k];
+  __syncthreads();
 #pragma unroll
-  for (int k = 0; k < 8; k++) x[k] = srow[rsw(64 * b + u0 + 8 * k)];
-  radix8_inv(x, tw, 1024 + 8 * r + b, 2048 + 16 * r + 2 * b, 4096 + 32 * r + 4 * b, q);
-  row_sync(bar);
+  for (int k = 0; k < 16; k++) x[k] = sm[rpos(b, k, u)];
+  {
+    uint2 w[16];
+    tw_radix16(tw, 256 + 16 * r + b, w);
+    radix16_fwd(x, w, q);
+  }
 #pragma unroll
-  for (int k = 0; k < 8; k++) srow[rsw(64 * b + u0 + 8 * k)] = x[k];
-  row_sync(bar);
-#pragma unroll
-  for (int k = 0; k < 8; k++) x[k] = srow[rsw(t + 64 * k)];
-  radix8_inv(x, tw, 128 + r, 256 + 2 * r, 512 + 4 * r, q);
+  for (int k = 0; k < 16; k++) sm[rpos(b, k, u)] = x[k];
+  __syncwarp();
+  group_ld(sm, t, x);
+  {
+    uint2 w[16];
+    tw_radix16_last(tw, r, t, w);
+    radix16_fwd(x, w, q);
+  }
+  group_st(sm, t, x);
+  __syncwarp();
+  chunk_ld(sm, t, x);
 }
 
-__device__ __forceinline__ void ld8(const uint32_t *p, uint32_t *x) {
-  const uint4 *v = reinterpret_cast<const uint4 *>(p);
-  const uint4 a = __ldg(v), b = __ldg(v + 1);
-  x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
-  x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+// The 12 row stages of the inverse transform: x in chunk order -> row order.
+__device__ __forceinline__ void row_inv(uint32_t *x, uint32_t *sm, const uint2 *tw, int r, int t, uint32_t q) {
+  const int b = t >> 4, u = t & 15;
+  chunk_st(sm, t, x);
+  __syncwarp();
+  group_ld(sm, t, x);
+  {
+    uint2 w[16];
+    tw_radix16_last(tw, r, t, w);
+    radix16_inv(x, w, q);
+  }
+  group_st(sm, t, x);
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < 16; k++) x[k] = sm[rpos(b, k, u)];
+  {
+    uint2 w[16];
+    tw_radix16(tw, 256 + 16 * r + b, w);
+    radix16_inv(x, w, q);
+  }
+#pragma unroll
+  for (int k = 0; k < 16; k++) sm[rpos(b, k, u)] = x[k];
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < 16; k++) x[k] = sm[rpos(k, b, u)];
+  {
+    uint2 w[16];
+    tw_radix16(tw, 16 + r, w);
+    radix16_inv(x, w, q);
+  }
 }
-__device__ __forceinline__ void st8(uint32_t *p, const uint32_t *x) {
-  uint4 *v = reinterpret_cast<uint4 *>(p);
-  v[0] = make_uint4(x[0], x[1], x[2], x[3]);
-  v[1] = make_uint4(x[4], x[5], x[6], x[7]);
+
+// 16 words of a row in chunk order; p = row start + chunk_off(t)
+__device__ __forceinline__ void ld_chunks(const uint32_t *p, uint32_t *x) {
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const uint4 v = __ldg(reinterpret_cast<const uint4 *>(p + 64 * i));
+    x[4 * i] = v.x; x[4 * i + 1] = v.y; x[4 * i + 2] = v.z; x[4 * i + 3] = v.w;
+  }
+}
+__device__ __forceinline__ void st_chunks(uint32_t *p, const uint32_t *x) {
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+    *reinterpret_cast<uint4 *>(p + 64 * i) = make_uint4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]);
 }
 
 }  // namespace chd

@@ -416,48 +416,27 @@ void chd_graph_destroy(chd_graph *g);
  * tensor-core wait that ran out. */
 #define CHD_BCONV_CUDA_CORE 0
 #define CHD_BCONV_TENSOR_CORE 1
-#define CHD_BCONV_AUTO 2 /* chd_set_ks_engine only: autotuned per launch shape */
-/* chd_set_ks_engine only: the tensor-core column pass on 256-thread tiles
- * (8 coefficients per thread, twice the warps per SM) for ModUp / ModDown
- * with at most 12 sources; larger ones use CHD_BCONV_TENSOR_CORE */
-#define CHD_BCONV_TENSOR_CORE_WIDE 3
+#define CHD_BCONV_AUTO 2             /* chd_set_ks_engine only */
+#define CHD_BCONV_TENSOR_CORE_WIDE 3 /* chd_set_ks_engine only */
 int chd_bconv_batch(chd_context *ctx, int engine, int npoly, const int32_t *xt_dev, const int *src_gidx, int K,
                     const int *dst_gidx, int M, uint32_t *out_dev);
 
-/* Engine of the base conversion inside every ModUp / ModDown of the fused
- * key-switching, rescaling and bootstrapping paths (HMult, relinearize,
- * rotations, hoisted rotations, linear transforms, ModDown epilogues):
- * CHD_BCONV_CUDA_CORE (int64 multiply-adds), CHD_BCONV_TENSOR_CORE (the
- * column pass issues INT8 byte-limb MMAs on the tcgen05 tensor cores with
- * int32 accumulation in TMEM, 128-thread tiles) or
- * CHD_BCONV_TENSOR_CORE_WIDE (the same on 256-thread tiles).  All give
- * bit-identical residues.
- * CHD_BCONV_AUTO autotunes: the first column pass of each launch shape
- * (device, sources, jobs, targets) outside a stream capture times the
- * three with each split of the targets over 1, 2, 4 or the heuristic
- * number of CTAs per column tile (one host synchronisation per shape and
- * process) and keeps the fastest (a tensor-core candidate within 3 % of a
- * faster CUDA-core one, as it shares an SM better with the other stream's
- * kernels); an untuned shape met during a capture
- * uses the tensor cores with the heuristic split.  No reference counterpart (the reference has one CUDA-core
- * implementation, src/core/ModSwitch.cu:23-171).  chd_get_ks_engine returns
- * the engine, -1 for a null context. */
+/* Engine of the fused key-switching, rescaling and bootstrapping paths.  All
+ * four values are accepted and give bit-identical residues.  At N = 2^16 one
+ * column pass (INT8 byte-limb MMAs in registers, exact int32 accumulation)
+ * serves every ModUp / ModDown whatever the engine; below it the base
+ * conversion runs on the CUDA cores.  CHD_BCONV_AUTO still times the register
+ * variants of the hoisted rotations and of the plaintext accumulation on the
+ * first launch of each shape outside a stream capture (one host
+ * synchronisation per shape and process).  No reference counterpart (the
+ * reference has one CUDA-core implementation, src/core/ModSwitch.cu:23-171).
+ * chd_get_ks_engine returns the engine, -1 for a null context. */
 int chd_set_ks_engine(chd_context *ctx, int engine);
 int chd_get_ks_engine(const chd_context *ctx);
-/* The autotuner's choices so far (no reference counterpart): per launch
- * shape six ints (device, largest source count K, jobs, largest target
- * count M, engine: 0 CUDA cores, 1 tensor cores, 3 / 4 tensor cores on
- * 256-thread tiles at 80 / 128 registers, target split) into out
- * (capacity cap shapes);
- * returns the number of shapes tuned in this process. */
+/* Shapes of the column pass (six ints each) and of the key-switch row pass
+ * (five ints each) whose variant was chosen by timing: none, each pass has
+ * one variant.  Both return 0 and write nothing. */
 int chd_ks_tuned_shapes(int *out, int cap);
-/* The same for the key-switch row pass (no reference counterpart): with
- * CHD_BCONV_AUTO its first launch of each shape times the variant that
- * loads each digit's key words and the next digit's ModUp row ahead (2 CTAs
- * per SM) against the one that loads where it computes at 3 and at 4 CTAs
- * per SM; five ints per shape (device, ciphertexts, largest row count of
- * the launch, mode, variant: 0 loads where used at 3 CTAs per SM, 1 loads
- * ahead, 2 loads where used at 4); returns the count. */
 int chd_ks_rows_tuned_shapes(int *out, int cap);
 /* Two-stream key switching (no reference counterpart; on by default, the
  * environment variable CHD_SPLIT_STREAMS=0 turns it off at context
