@@ -270,7 +270,7 @@ Status Context::decode(int level, double scale, const uint32_t *pt_dev, int num_
   cr.Q_lo = static_cast<uint64_t>(Q);
   cr.Q_hi = static_cast<uint64_t>(Q >> 64);
   cr.rows = tot;
-  for_row_batches(rows, [&](const RowBatch &rb) { launch_ntt_inv(rb, P->log_n, stream); });
+  for_row_batches(rows, [&](RowBatch &rb) { launch_ntt_inv(rb, P->log_n, stream); });
   const int th = 256;
   k_crt_decode<<<(num_slots + th - 1) / th, th, 0, stream>>>(y, n, gap, num_slots, scale, cr, d);
   k_bit_reverse<<<(num_slots + th - 1) / th, th, 0, stream>>>(d, e, num_slots, log2_exact(num_slots));

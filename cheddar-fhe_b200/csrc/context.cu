@@ -932,8 +932,10 @@ Status Context::ntt(const NP &np, uint32_t *data, bool mont, int count, size_t s
   std::vector<int> g(tot);
   P->gidx(np, g.data());
   std::vector<RowDesc> rows;
-  for (int c = 0; c < count; c++)
-    for (int i = 0; i < tot; i++) {
+  for (int c0 = 0; c0 < count; c0 += 2)  // limbs of one prime side by side: the row phase takes them in pairs
+    for (int k = 0; k < 2 * tot; k++) {
+      const int i = k >> 1, c = c0 + (k & 1);
+      if (c == count) continue;
       RowDesc r{};
       r.src = r.dst = data + c * stride + static_cast<size_t>(i) * n;
       r.tw = tw(g[i]);
@@ -943,11 +945,11 @@ Status Context::ntt(const NP &np, uint32_t *data, bool mont, int count, size_t s
       rows.push_back(r);
     }
   return alternate_row_batches(rows, count > 1 && stride >= static_cast<size_t>(tot) * n,
-                               [&](const RowBatch &rb, cudaStream_t s) { launch_ntt_fwd(rb, P->log_n, s); }, "ntt");
+                               [&](RowBatch &rb, cudaStream_t s) { launch_ntt_fwd(rb, P->log_n, s); }, "ntt");
 }
 
 Status Context::alternate_row_batches(const std::vector<RowDesc> &rows, bool disjoint,
-                                      const std::function<void(const RowBatch &, cudaStream_t)> &launch,
+                                      const std::function<void(RowBatch &, cudaStream_t)> &launch,
                                       const char *what) {
   // more rows than one launch takes: the launches alternate between the
   // context stream and aux_stream (forked and joined as in fork_halves), so
@@ -959,13 +961,13 @@ Status Context::alternate_row_batches(const std::vector<RowDesc> &rows, bool dis
   const bool split = split_streams && aux_stream != nullptr && disjoint &&
                      static_cast<int>(rows.size()) > kAltRows;
   if (!split) {
-    for_row_batches(rows, [&](const RowBatch &rb) { launch(rb, stream); });
+    for_row_batches(rows, [&](RowBatch &rb) { launch(rb, stream); });
     return check_cuda(what);
   }
   CHD_CHECK(cudaEventRecord(ev_fork, stream) == cudaSuccess && cudaStreamWaitEvent(aux_stream, ev_fork, 0) == cudaSuccess,
             kErrCuda, "stream fork failed");
   int k = 0;
-  for_row_batches(rows, [&](const RowBatch &rb) { launch(rb, (k++ & 1) ? aux_stream : stream); }, kAltRows);
+  for_row_batches(rows, [&](RowBatch &rb) { launch(rb, (k++ & 1) ? aux_stream : stream); }, kAltRows);
   const bool joined =
       cudaEventRecord(ev_join, aux_stream) == cudaSuccess && cudaStreamWaitEvent(stream, ev_join, 0) == cudaSuccess;
   CHD_CHECK(joined, kErrCuda, "stream join failed");
@@ -977,8 +979,10 @@ Status Context::intt(const NP &np, uint32_t *data, bool mont, int count, size_t 
   std::vector<int> g(tot);
   P->gidx(np, g.data());
   std::vector<RowDesc> rows;
-  for (int c = 0; c < count; c++)
-    for (int i = 0; i < tot; i++) {
+  for (int c0 = 0; c0 < count; c0 += 2)  // limbs of one prime side by side: the row phase takes them in pairs
+    for (int k = 0; k < 2 * tot; k++) {
+      const int i = k >> 1, c = c0 + (k & 1);
+      if (c == count) continue;
       RowDesc r{};
       r.src = r.dst = data + c * stride + static_cast<size_t>(i) * n;
       r.tw = itw(g[i]);
@@ -987,7 +991,7 @@ Status Context::intt(const NP &np, uint32_t *data, bool mont, int count, size_t 
       rows.push_back(r);
     }
   return alternate_row_batches(rows, count > 1 && stride >= static_cast<size_t>(tot) * n,
-                               [&](const RowBatch &rb, cudaStream_t s) { launch_ntt_inv(rb, P->log_n, s); }, "intt");
+                               [&](RowBatch &rb, cudaStream_t s) { launch_ntt_inv(rb, P->log_n, s); }, "intt");
 }
 
 Status Context::bconv(const int32_t *xt, int K, const int32_t *table, const int *dst_gidx, int M, uint32_t *out) {
@@ -1144,7 +1148,7 @@ Status Context::modup_many(int level, int count, const uint32_t *const *src, uin
       d.flags = kCentre;
       rows.push_back(d);
     }
-  for_row_batches(rows, [&](const RowBatch &rb) { launch_ntt_inv(rb, P->log_n, stream); });
+  for_row_batches(rows, [&](RowBatch &rb) { launch_ntt_inv(rb, P->log_n, stream); });
   // 2. own primes copied, others base-converted
   BConvBatch b{};
   b.primes = d_primes;
@@ -1190,7 +1194,7 @@ Status Context::modup_many(int level, int count, const uint32_t *const *src, uin
         rows.push_back(d);
       }
     }
-  for_row_batches(rows, [&](const RowBatch &rb) { launch_ntt_fwd(rb, P->log_n, stream); });
+  for_row_batches(rows, [&](RowBatch &rb) { launch_ntt_fwd(rb, P->log_n, stream); });
   return check_cuda("modup");
 }
 
@@ -1205,8 +1209,10 @@ Status Context::modup_fused(int level, int count, const uint32_t *const *src, ui
   std::vector<int> g(tot);
   P->gidx(np, g.data());
   std::vector<RowDesc> rows;
-  for (int c = 0; c < count; c++)
-    for (int r = 0; r < nq; r++) {
+  for (int c0 = 0; c0 < count; c0 += 2)
+    for (int k = 0; k < 2 * nq; k++) {
+      const int r = k >> 1, c = c0 + (k & 1);
+      if (c == count) continue;
       RowDesc d{};
       d.src = src[c] + static_cast<size_t>(r) * n;
       d.dst = rows_out + (static_cast<size_t>(c) * nq + r) * n;
@@ -1214,7 +1220,7 @@ Status Context::modup_fused(int level, int count, const uint32_t *const *src, ui
       d.q = P->primes[g[r]];
       rows.push_back(d);
     }
-  for_row_batches(rows, [&](const RowBatch &rb) { launch_ntt_inv_rows(rb, P->log_n, stream); });
+  for_row_batches(rows, [&](RowBatch &rb) { launch_ntt_inv_rows(rb, P->log_n, stream); });
   MSColBatch b{};
   b.tw = d_tw;
   b.itw = d_itw;
@@ -1253,19 +1259,17 @@ Status Context::modup_fused(int level, int count, const uint32_t *const *src, ui
   launch_modswitch_cols(b, P->log_n, stream);
   rows.clear();
   for (int c = 0; c < count; c++)
-    for (int i = 0; i < m.beta; i++) {
-      const int s = m.dig_s[i], e = m.dig_e[i];
-      if (e <= 0) continue;
-      for (int r = 0; r < tot; r++) {
-        if (r >= s && r < e) continue;
+    for (int i0 = 0; i0 < m.beta; i0 += 2)
+      for (int k = 0; k < 2 * tot; k++) {
+        const int r = k >> 1, i = i0 + (k & 1);
+        if (i == m.beta || m.dig_e[i] <= 0 || (r >= m.dig_s[i] && r < m.dig_e[i])) continue;
         RowDesc d{};
         d.src = d.dst = dst[c][i] + static_cast<size_t>(r) * n;
         d.tw = tw(g[r]);
         d.q = P->primes[g[r]];
         rows.push_back(d);
       }
-    }
-  for_row_batches(rows, [&](const RowBatch &rb) { launch_ntt_fwd_rows(rb, P->log_n, stream); });
+  for_row_batches(rows, [&](RowBatch &rb) { launch_ntt_fwd_rows(rb, P->log_n, stream); });
   return check_cuda("modup");
 }
 
@@ -1398,9 +1402,13 @@ Status Context::key_switch_fused_pipeline(const int *levels, int count, const KS
   auto MU = [&](int c, int b) { return mu + (o_mu[c] + static_cast<size_t>(b) * shapes[levels[c]].tot) * N; };
   // 1. ModUp INTT row phase of the key-switched input (a1 a2 / ax / rx)
   std::vector<RowDesc> rows;
-  for (int c = 0; c < count; c++) {
-    const Shape &sh = shapes[levels[c]];
-    for (int r = 0; r < sh.nq; r++) {
+  for (int c0 = 0, cn; c0 < count; c0 = cn) {
+    // two ciphertexts of one level side by side: the row phase pairs limbs of
+    // one prime
+    cn = c0 + (c0 + 1 < count && levels[c0 + 1] == levels[c0] ? 2 : 1);
+    const Shape &sh = shapes[levels[c0]];
+    for (int k = 0; k < (cn - c0) * sh.nq; k++) {
+      const int r = k / (cn - c0), c = c0 + k % (cn - c0);
       RowDesc d{};
       const size_t o = static_cast<size_t>(r) * N;
       d.src = (in[c].mode == 2 ? in[c].a2 : in[c].a1) + o;
@@ -1416,7 +1424,7 @@ Status Context::key_switch_fused_pipeline(const int *levels, int count, const KS
     }
   }
   int nl = 0, t0 = timer_mark();
-  for_row_batches(rows, [&](const RowBatch &rb) {
+  for_row_batches(rows, [&](RowBatch &rb) {
     launch_ntt_inv_rows(rb, P->log_n, stream);
     nl++;
   });
@@ -1583,10 +1591,10 @@ Status Context::key_switch_fused_pipeline(const int *levels, int count, const KS
   for (int c = 0; c < count; c++) {
     const Shape &sh = shapes[levels[c]];
     const MDPlan &pl = sh.pl;
-    for (int p = 0; p < 2; p++) {
-      const uint32_t *src = acc + (o_acc[c] + static_cast<size_t>(p) * sh.tot) * N;
-      uint32_t *dst = p == 0 ? in[c].out_b : in[c].out_a;
-      for (int y = 0; y < pl.dst_len; y++) {
+    for (int y = 0; y < pl.dst_len; y++) {
+      for (int p = 0; p < 2; p++) {
+        const uint32_t *src = acc + (o_acc[c] + static_cast<size_t>(p) * sh.tot) * N;
+        uint32_t *dst = p == 0 ? in[c].out_b : in[c].out_a;
         RowDesc d{};
         d.src = d.dst = dst + static_cast<size_t>(y) * N;
         d.tw = tw(pl.gd[y]);
@@ -1607,7 +1615,7 @@ Status Context::key_switch_fused_pipeline(const int *levels, int count, const KS
   }
   nl = 0;
   t0 = timer_mark();
-  for_row_batches(rows, [&](const RowBatch &rb) {
+  for_row_batches(rows, [&](RowBatch &rb) {
     launch_ntt_fwd_rows(rb, P->log_n, stream);
     nl++;
   });
@@ -1692,8 +1700,10 @@ Status Context::moddown_pipeline(int level, MDType type, const uint32_t *const *
   CHD_CHECK(xt, kErrAlloc, "moddown: scratch allocation failed");
   std::vector<RowDesc> rows;
   const bool fused = P->log_n == 16;
-  for (int p = 0; p < npoly; p++)
-    for (int i = 0; i < src_len; i++) {
+  for (int p0 = 0; p0 < npoly; p0 += 2)
+    for (int k = 0; k < 2 * src_len; k++) {
+      const int i = k >> 1, p = p0 + (k & 1);
+      if (p == npoly) continue;
       const int gg = gs[srows[i]];
       RowDesc d{};
       d.src = src[p] + static_cast<size_t>(srows[i]) * n;
@@ -1705,7 +1715,7 @@ Status Context::moddown_pipeline(int level, MDType type, const uint32_t *const *
       rows.push_back(d);
     }
   if (fused) {
-    for_row_batches(rows, [&](const RowBatch &rb) { launch_ntt_inv_rows(rb, P->log_n, stream); });
+    for_row_batches(rows, [&](RowBatch &rb) { launch_ntt_inv_rows(rb, P->log_n, stream); });
     MSColBatch b{};
     b.tw = d_tw;
     b.itw = d_itw;
@@ -1735,7 +1745,7 @@ Status Context::moddown_pipeline(int level, MDType type, const uint32_t *const *
     }
     launch_modswitch_cols(b, P->log_n, stream);
   } else {
-    for_row_batches(rows, [&](const RowBatch &rb) { launch_ntt_inv(rb, P->log_n, stream); });
+    for_row_batches(rows, [&](RowBatch &rb) { launch_ntt_inv(rb, P->log_n, stream); });
     BConvBatch b{};
     b.primes = d_primes;
     b.qinvs = d_qinv;
@@ -1760,8 +1770,10 @@ Status Context::moddown_pipeline(int level, MDType type, const uint32_t *const *
   const int src2_start = nd.ter - nn.ter, src2_end = src2_start + nn.q();
   const int src2_off = std::max(0, ns.ter - nd.ter);
   rows.clear();
-  for (int p = 0; p < npoly; p++)
-    for (int y = 0; y < dst_len; y++) {
+  for (int p0 = 0; p0 < npoly; p0 += 2)
+    for (int k = 0; k < 2 * dst_len; k++) {
+      const int y = k >> 1, p = p0 + (k & 1);
+      if (p == npoly) continue;
       RowDesc d{};
       d.src = d.dst = dst[p] + static_cast<size_t>(y) * n;
       d.tw = tw(gd[y]);
@@ -1779,9 +1791,9 @@ Status Context::moddown_pipeline(int level, MDType type, const uint32_t *const *
       rows.push_back(d);
     }
   if (fused)
-    for_row_batches(rows, [&](const RowBatch &rb) { launch_ntt_fwd_rows(rb, P->log_n, stream); });
+    for_row_batches(rows, [&](RowBatch &rb) { launch_ntt_fwd_rows(rb, P->log_n, stream); });
   else
-    for_row_batches(rows, [&](const RowBatch &rb) { launch_ntt_fwd(rb, P->log_n, stream); });
+    for_row_batches(rows, [&](RowBatch &rb) { launch_ntt_fwd(rb, P->log_n, stream); });
   return check_cuda("moddown");
 }
 

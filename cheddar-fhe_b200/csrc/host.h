@@ -6,6 +6,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <map>
 #include <memory>
@@ -431,7 +432,7 @@ class Context {
   // the context stream and aux_stream when there are several batches of
   // disjoint rows
   Status alternate_row_batches(const std::vector<RowDesc> &rows, bool disjoint,
-                               const std::function<void(const RowBatch &, cudaStream_t)> &launch, const char *what);
+                               const std::function<void(RowBatch &, cudaStream_t)> &launch, const char *what);
   Status bconv(const int32_t *xt, int K, const int32_t *table, const int *dst_gidx, int M, uint32_t *out);
   // BConv of npoly polynomials ([npoly][K][N] -> [npoly][M][N]) with the
   // host table T[m][k] (centred, Montgomery q-hat R^2): engine 0 on the CUDA
@@ -605,7 +606,8 @@ void for_row_batches(const std::vector<RowDesc> &rows, F &&launch, int cap = kMa
   cap = cap < 1 || cap > kMaxRows ? kMaxRows : cap;
   const int total = static_cast<int>(rows.size());
   const int nbat = (total + cap - 1) / cap;
-  const int per = nbat > 0 ? (total + nbat - 1) / nbat : cap;
+  // an even number, so that pairs of one prime stay together
+  const int per = nbat > 0 ? std::min(cap, ((total + nbat - 1) / nbat + 1) & ~1) : cap;
   RowBatch rb;
   rb.count = 0;
   for (const RowDesc &r : rows) {

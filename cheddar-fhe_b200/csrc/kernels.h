@@ -42,6 +42,7 @@ constexpr int kMaxRows = 256;
 
 struct RowBatch {
   int count;
+  uint16_t first[kMaxRows + 1];  // set by the row-phase launches: first limb of each CTA's group
   RowDesc rows[kMaxRows];
 };
 static_assert(sizeof(RowBatch) + 16 <= 32764, "row batch beyond the kernel parameter limit");
@@ -49,13 +50,13 @@ static_assert(sizeof(RowBatch) + 16 <= 32764, "row batch beyond the kernel param
 // Forward negacyclic NTT (bit-reversed output) of `count` limbs.
 // Column phase then row phase for log_n = 16; a single-kernel shared-memory
 // transform for log_n <= 15.  In-place allowed (dst == src).
-void launch_ntt_fwd(const RowBatch &rb, int log_n, cudaStream_t s);
+void launch_ntt_fwd(RowBatch &rb, int log_n, cudaStream_t s);
 // Row phase only / column phase only (used by fused pipelines and tests)
 void launch_ntt_fwd_cols(const RowBatch &rb, int log_n, cudaStream_t s);
-void launch_ntt_fwd_rows(const RowBatch &rb, int log_n, cudaStream_t s);
+void launch_ntt_fwd_rows(RowBatch &rb, int log_n, cudaStream_t s);
 // Inverse NTT (bit-reversed input); epilogue x * c0, canonical or centred
 // (kCentre).  tw must point at the inverse twiddle table.
-void launch_ntt_inv(const RowBatch &rb, int log_n, cudaStream_t s);
+void launch_ntt_inv(RowBatch &rb, int log_n, cudaStream_t s);
 
 // Base conversion of one job: out[m][n] = (sum_k xt[k][n] * T[m][k]) * 2^-32
 // mod p_m.  xt holds K consecutive centred limbs; destination limb m is
@@ -178,7 +179,7 @@ struct MSColBatch {
 };
 static_assert(sizeof(MSColBatch) + 16 <= 32764, "column-pass batch beyond the kernel parameter limit");
 void launch_modswitch_cols(const MSColBatch &b, int log_n, cudaStream_t s);
-void launch_ntt_inv_rows(const RowBatch &rb, int log_n, cudaStream_t s);
+void launch_ntt_inv_rows(RowBatch &rb, int log_n, cudaStream_t s);
 
 // Fused key-switching row pass (N = 2^16), see keyswitch.cu.  Modes:
 //   0 HMult:       own ModUp value a1 a2, d0 = b1 b2, d1 = b1 a2 + a1 b2

@@ -28,6 +28,8 @@ namespace {
 // then below 2q, is brought back below q (one instruction; q 2^32 is a
 // multiple of q).  One Montgomery reduction at the end replaces one per
 // product.
+constexpr int kMaxDigits = 8;  // KSRowsLevel::kb
+
 __device__ __forceinline__ void acc_fold(uint64_t &s, uint32_t q) {
   const uint32_t hi = reduce2q(static_cast<uint32_t>(s >> 32), q);
   s = (static_cast<uint64_t>(hi) << 32) | static_cast<uint32_t>(s);
@@ -40,8 +42,111 @@ __device__ __forceinline__ uint32_t acc_reduce(uint64_t s, uint32_t q, int32_t q
   return min(r, r + q);
 }
 
-__global__ void __launch_bounds__(kRowThreads, 2) k_ks_rows(const __grid_constant__ KSRowsDesc d) {
-  __shared__ __align__(16) uint32_t sm[2][kRowLen];
+// Inner product and P (d0, d1) of one row, four coefficients at a time, for
+// beta digits whose canonical ModUp rows lie in the row buffers (beta known
+// at compile time up to 4, so that the key words of all digits can be in
+// flight together and their pointers stay in registers; B = 0: any beta).
+template <int B>
+__device__ __forceinline__ void inner_product(const KSRowsCt &c, const KSRowsLevel &L, uint32_t *sm, int j, int mode,
+                                              size_t off, size_t koff, uint32_t q, int32_t qi, int t) {
+  const bool is_q = j < L.nq, with_p = is_q && c.b1 != nullptr;
+  const int own = L.own_digit[j], di = L.drop_idx[j], beta = B ? B : L.beta;
+  const uint32_t *kb[B ? B : 1], *ka[B ? B : 1];
+#pragma unroll
+  for (int i = 0; i < B; i++) {
+    kb[i] = L.kb[i] + koff;
+    ka[i] = L.ka[i] + koff;
+  }
+#pragma unroll 1
+  for (int e = 0; e < 4; e++) {
+    auto ld4 = [&](const uint32_t *p, uint32_t *x) {
+      const uint4 v4 = __ldg(reinterpret_cast<const uint4 *>(p + 64 * e));
+      x[0] = v4.x; x[1] = v4.y; x[2] = v4.z; x[3] = v4.w;
+    };
+    uint64_t sb[4] = {0, 0, 0, 0}, sa[4] = {0, 0, 0, 0};
+    uint32_t vo[4] = {0, 0, 0, 0};
+    if (is_q) {
+      // the own digit's ModUp value is the key-switched input; P * (d0, d1):
+      // HMult d0 = b1 b2, d1 = b1 a2 + a1 b2; MultKey d0 = bx; Relinearize
+      // d0 = bx, d1 = ax.  Without b1: the bare inner product.
+      const uint64_t pp = L.p_prod[j];
+      uint32_t a1[4], a2[4], b1[4], b2[4];
+      ld4(c.a1 + off, a1);
+      if (mode != 1) ld4(c.a2 + off, a2);
+      if (with_p) ld4(c.b1 + off, b1);
+      if (mode == 0) {
+        ld4(c.b2 + off, b2);
+        const uint32_t qneg = 0u - static_cast<uint32_t>(qi);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          vo[k] = mont_mul(a1[k], a2[k], q, qi);
+          sb[k] = pp * mont_mul(b1[k], b2[k], q, qi);
+          sa[k] = pp * mont_mac2(b1[k], a2[k], a1[k], b2[k], q, qneg);
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          vo[k] = mode == 1 ? a1[k] : a2[k];
+          if (with_p) sb[k] = pp * b1[k];
+          if (with_p && mode == 2) sa[k] = pp * a1[k];
+        }
+      }
+    }
+    auto digit = [&](int i, const uint32_t *pb, const uint32_t *pa) {
+      uint32_t b4[4], a4[4];
+      ld4(pb, b4);
+      ld4(pa, a4);
+      uint4 v4 = make_uint4(vo[0], vo[1], vo[2], vo[3]);
+      if (own != i) v4 = chunk_ld4(sm + i * kRowBuf, t, e);
+      const uint32_t v[4] = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        sb[k] += static_cast<uint64_t>(v[k]) * b4[k];
+        sa[k] += static_cast<uint64_t>(v[k]) * a4[k];
+      }
+      if (i & 1) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          acc_fold(sb[k], q);
+          acc_fold(sa[k], q);
+        }
+      }
+    };
+    if (B) {
+#pragma unroll
+      for (int i = 0; i < B; i++) digit(i, kb[i], ka[i]);
+    } else {
+      for (int i = 0; i < beta; i++) digit(i, L.kb[i] + koff, L.ka[i] + koff);
+    }
+    uint32_t ob[4], oa[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      ob[k] = acc_reduce(sb[k], q, qi);
+      oa[k] = acc_reduce(sa[k], q, qi);
+    }
+    const uint4 b4 = make_uint4(ob[0], ob[1], ob[2], ob[3]), a4 = make_uint4(oa[0], oa[1], oa[2], oa[3]);
+    if (di < 0) {
+      *reinterpret_cast<uint4 *>(c.acc_b + off + 64 * e) = b4;
+      *reinterpret_cast<uint4 *>(c.acc_a + off + 64 * e) = a4;
+    } else {
+      // this thread has read chunk e of every digit
+      chunk_st4(sm, t, e, b4);
+      chunk_st4(sm + kRowBuf, t, e, a4);
+    }
+  }
+}
+
+// What bounds it: integer issue (61 % of cycles, the multiplier 64 % busy) and
+// the latency of its loads, so occupancy decides.  Each digit's transformed
+// row waits in shared memory and the inner product runs over four
+// coefficients at a time, so that 64 registers suffice and four CTAs share an
+// SM.  8 multiplications at level 22, one stream: 198 us; with 64-bit
+// accumulators of the whole row in registers (128, two CTAs) 235, with 32-bit
+// ones (80 and spilled, three CTAs) 224; the 128 x 512 form before it 218
+// with three stages fewer.  Two digits per transform (sharing twiddles, 80
+// registers, three CTAs) 227; L2 prefetch of the key rows no gain.
+__global__ void __launch_bounds__(kRowThreads, 4) k_ks_rows(const __grid_constant__ KSRowsDesc d) {
+  extern __shared__ __align__(16) uint32_t sm[];  // one row buffer per digit, at least two
   // grid (count, 16, max_rows): the ciphertexts sharing one key row are
   // neighbours in launch order, so the key row comes from HBM once
   const int j = blockIdx.z;
@@ -54,118 +159,55 @@ __global__ void __launch_bounds__(kRowThreads, 2) k_ks_rows(const __grid_constan
   const uint2 *tw = d.tw + (static_cast<size_t>(g) << 16);
   const int t = threadIdx.x, r = blockIdx.y;
   const size_t row = static_cast<size_t>(j) * 65536 + r * kRowLen;
+  const int own = L.own_digit[j], beta = L.beta;
+  // ---- ModUp NTT rows: each digit's row stays in its buffer
+  for (int i = 0; i < beta; i++) {
+    if (own == i) continue;
+    const uint32_t *src = c.mu[i] + row;
+    uint32_t v[1][16];
+    uint32_t *bufs[1] = {sm + i * kRowBuf};
+#pragma unroll
+    for (int k = 0; k < 16; k++) v[0][k] = src[t + 256 * k];
+    row_fwd_group<1>(v, false, bufs, tw, r, t, q);
+#pragma unroll
+    for (int k = 0; k < 16; k++) v[0][k] = reduce2q(v[0][k], q);
+    group_st(bufs[0], t, v[0]);
+  }
+  __syncwarp();  // chunks are read back within the half-warp that wrote them
+  // ---- inner product and P (d0, d1)
   const size_t off = row + chunk_off(t);  // input rows share the accumulator row index for q primes
   const size_t koff = static_cast<size_t>(L.key_row[j]) * 65536 + r * kRowLen + chunk_off(t);
-  const bool is_q = j < L.nq;
-  const int mode = d.mode;
-  uint64_t sb[16], sa[16];
-#pragma unroll
-  for (int k = 0; k < 16; k++) sb[k] = sa[k] = 0;
-  const int own = L.own_digit[j];
-  int buf = 0;
-  for (int i = 0; i < L.beta; i++) {
-    uint32_t v[16];
-    if (own == i) {
-      // own primes of the digit: the ModUp value is the key-switched input
-      ld_chunks((mode == 2 ? c.a2 : c.a1) + off, v);
-      if (mode == 0) {
-        uint32_t y[16];
-        ld_chunks(c.a2 + off, y);
-#pragma unroll
-        for (int k = 0; k < 16; k++) v[k] = mont_mul(v[k], y[k], q, qi);
-      }
-    } else {
-      const uint32_t *src = c.mu[i] + row;
-#pragma unroll
-      for (int k = 0; k < 16; k++) v[k] = src[t + 256 * k];
-      row_fwd(v, sm[buf], tw, r, t, q);
-      buf ^= 1;
-#pragma unroll
-      for (int k = 0; k < 16; k++) v[k] = reduce2q(v[k], q);
-    }
-    const uint32_t *kb = L.kb[i] + koff, *ka = L.ka[i] + koff;
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-      const uint4 b4 = __ldg(reinterpret_cast<const uint4 *>(kb + 64 * e));
-      const uint4 a4 = __ldg(reinterpret_cast<const uint4 *>(ka + 64 * e));
-      const uint32_t kbv[4] = {b4.x, b4.y, b4.z, b4.w}, kav[4] = {a4.x, a4.y, a4.z, a4.w};
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        sb[4 * e + k] += static_cast<uint64_t>(v[4 * e + k]) * kbv[k];
-        sa[4 * e + k] += static_cast<uint64_t>(v[4 * e + k]) * kav[k];
-      }
-    }
-    if (i & 1) {
-#pragma unroll
-      for (int k = 0; k < 16; k++) {
-        acc_fold(sb[k], q);
-        acc_fold(sa[k], q);
-      }
-    }
-  }
-  if (is_q && c.b1 != nullptr) {
-    // P * (d0, d1): HMult d0 = b1 b2, d1 = b1 a2 + a1 b2; MultKey d0 = bx;
-    // Relinearize d0 = bx, d1 = ax.  Without b1: the bare inner product.
-    const uint64_t pp = L.p_prod[j];
-    const uint32_t qneg = 0u - static_cast<uint32_t>(qi);
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-      auto ld4 = [&](const uint32_t *p, uint32_t *x) {
-        const uint4 v4 = __ldg(reinterpret_cast<const uint4 *>(p + off + 64 * e));
-        x[0] = v4.x; x[1] = v4.y; x[2] = v4.z; x[3] = v4.w;
-      };
-      uint32_t b1[4];
-      ld4(c.b1, b1);
-      if (mode == 0) {
-        uint32_t b2[4], a1[4], a2[4];
-        ld4(c.b2, b2);
-        ld4(c.a1, a1);
-        ld4(c.a2, a2);
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-          sb[4 * e + k] += pp * mont_mul(b1[k], b2[k], q, qi);
-          sa[4 * e + k] += pp * mont_mac2(b1[k], a2[k], a1[k], b2[k], q, qneg);
-        }
-      } else {
-#pragma unroll
-        for (int k = 0; k < 4; k++) sb[4 * e + k] += pp * b1[k];
-        if (mode == 2) {
-          uint32_t a1[4];
-          ld4(c.a1, a1);
-#pragma unroll
-          for (int k = 0; k < 4; k++) sa[4 * e + k] += pp * a1[k];
-        }
-      }
-    }
-  }
-  uint32_t ob[16], oa[16];
-#pragma unroll
-  for (int k = 0; k < 16; k++) {
-    ob[k] = acc_reduce(sb[k], q, qi);
-    oa[k] = acc_reduce(sa[k], q, qi);
-  }
   const int di = L.drop_idx[j];
-  if (di < 0) {
-    st_chunks(c.acc_b + off, ob);
-    st_chunks(c.acc_a + off, oa);
-    return;
+  switch (beta) {
+    case 1: inner_product<1>(c, L, sm, j, d.mode, off, koff, q, qi, t); break;
+    case 2: inner_product<2>(c, L, sm, j, d.mode, off, koff, q, qi, t); break;
+    case 3: inner_product<3>(c, L, sm, j, d.mode, off, koff, q, qi, t); break;
+    case 4: inner_product<4>(c, L, sm, j, d.mode, off, koff, q, qi, t); break;
+    default: inner_product<0>(c, L, sm, j, d.mode, off, koff, q, qi, t); break;
   }
+  if (di < 0) return;
   // dropped prime: INTT row phase of both accumulators (ModDown's first step)
   const uint2 *itw = d.itw + (static_cast<size_t>(g) << 16);
   const size_t doff = static_cast<size_t>(di) * 65536 + r * kRowLen + t;
-  row_inv(ob, sm[buf], itw, r, t, q);
+#pragma unroll 1
+  for (int p = 0; p < 2; p++) {
+    uint32_t x[1][16];
+    uint32_t *bufs[1] = {sm + p * kRowBuf};
+    uint32_t *dst = (p == 0 ? c.drop_b : c.drop_a) + doff;
+    row_inv_stored<1>(x, false, bufs, itw, r, t, q);
 #pragma unroll
-  for (int k = 0; k < 16; k++) c.drop_b[doff + 256 * k] = ob[k];
-  row_inv(oa, sm[buf ^ 1], itw, r, t, q);
-#pragma unroll
-  for (int k = 0; k < 16; k++) c.drop_a[doff + 256 * k] = oa[k];
+    for (int k = 0; k < 16; k++) dst[256 * k] = x[0][k];
+  }
 }
 
 }  // namespace
 
 void launch_ks_rows(const KSRowsDesc &d, int log_n, cudaStream_t s) {
   if (d.count <= 0 || d.max_rows <= 0 || log_n != 16) return;
-  k_ks_rows<<<dim3(d.count, kLimbRows, d.max_rows), kRowThreads, 0, s>>>(d);
+  int bufs = 2;
+  for (int i = 0; i < d.nlv; i++) bufs = d.lv[i].beta > bufs ? d.lv[i].beta : bufs;
+  cudaFuncSetAttribute(k_ks_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDigits * kRowBuf * 4);
+  k_ks_rows<<<dim3(d.count, kLimbRows, d.max_rows), kRowThreads, bufs * kRowBuf * 4, s>>>(d);
 }
 
 }  // namespace chd

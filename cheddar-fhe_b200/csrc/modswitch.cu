@@ -71,19 +71,50 @@ __device__ __forceinline__ uint32_t join(int d0, int d1, int d2, int d3, uint32_
 }
 
 // KR: source rounds (sources tq + 4 i, i < KR; K <= 4 KR).  MINB CTAs per SM
-// (72, 80, 96 and 128 registers for KR = 1 .. 4, at most five words spilled):
+// (72, 80, 96 and 128 registers for KR = 1 .. 4, a few words spilled):
 // left alone the compiler takes 134 to 188, and the batch of 8 below slows
 // to 96 / 74 us; one step tighter spills and gives 94 / 76 us.
 //
 // Measured, 8 multiplications at level 22 on one stream: ModUp (24 jobs of
-// 8 sources and 24 targets) 90 us, ModDown + Rescale (16 jobs of 9 and 23)
-// 70 us; the 128 x 512 tcgen05 pass before it took 172 and 141 us.
+// 8 sources and 24 targets) 85 us, ModDown + Rescale (16 jobs of 9 and 23)
+// 68 us; the 128 x 512 tcgen05 pass before it took 172 and 141 us.
 template <int KR, int MINB>
 __global__ void __launch_bounds__(32 * kColWarps, MINB) k_modswitch_cols(const __grid_constant__ MSColBatch b) {
   const MSColJob &jb = b.jobs[blockIdx.y];
   const int lane = threadIdx.x & 31, tq = lane & 3;
   const int col = (blockIdx.x * kColWarps + (threadIdx.x >> 5)) * 8 + (lane >> 2);
   const int K = jb.K, M = jb.M;
+  // The fifteen twiddles of every source and target prime (the column stages
+  // use the first sixteen table entries): [group of four primes][pair of
+  // entries][prime], so that the four primes of a warp's 16-byte access lie
+  // in 64 contiguous bytes.  Read from the tables by every warp they cost
+  // four cache lines per access, and the pass filled the cache's data path
+  // (76 % of its peak; ModUp 88 -> 85 us, ModDown 70.5 -> 68).  With up to
+  // four sources there is too little work for the detour (a plaintext product
+  // and rescale at level 5: 24.0 us from the tables, 25.8 us staged).
+  constexpr bool kStaged = KR > 1;
+  extern __shared__ uint4 tws[];
+  uint4 *tws_dst = tws + 32 * KR;
+  for (int i = threadIdx.x; i < (kStaged ? 8 * (K + M) : 0); i += 32 * kColWarps) {
+    const int k = i >> 3, c = i & 7;
+    const bool src = k < K;
+    const int g = src ? jb.src_gidx[k] : jb.dst_gidx[k - K], x = src ? k : k - K;
+    const uint2 *tab = (src ? b.itw : b.tw) + (static_cast<size_t>(g) << 16);
+    (src ? tws : tws_dst)[32 * (x >> 2) + 4 * c + (x & 3)] = __ldg(reinterpret_cast<const uint4 *>(tab) + c);
+  }
+  if (kStaged) __syncthreads();
+  auto twiddles = [&](const uint4 *p, const uint2 *table, int g, uint2 *w) {
+    if (!kStaged) {
+      tw_radix16(table + (static_cast<size_t>(g) << 16), 1, w);
+      return;
+    }
+#pragma unroll
+    for (int c = 0; c < 8; c++) {
+      const uint4 v = p[4 * c];
+      w[2 * c] = make_uint2(v.x, v.y);
+      w[2 * c + 1] = make_uint2(v.z, v.w);
+    }
+  };
   // ---- INTT column stages, output constant, centring, offset
   uint32_t xs[KR][16];
 #pragma unroll
@@ -98,7 +129,7 @@ __global__ void __launch_bounds__(32 * kColWarps, MINB) k_modswitch_cols(const _
       uint2 w[16];
 #pragma unroll
       for (int e = 0; e < 16; e++) xs[i][e] = __ldg(src + e * kRowLen);
-      tw_radix16(b.itw + (static_cast<size_t>(g) << 16), 1, w);
+      twiddles(tws + 32 * i + (k & 3), b.itw, g, w);
       radix16_inv(xs[i], w, q);
 #pragma unroll
       for (int e = 0; e < 16; e++)
@@ -141,7 +172,7 @@ __global__ void __launch_bounds__(32 * kColWarps, MINB) k_modswitch_cols(const _
       v[e + 1] = join(lo[2], lo[3], hi[2], hi[3], p, pinv);
     }
     uint2 w[16];
-    tw_radix16(b.tw + (static_cast<size_t>(g) << 16), 1, w);
+    twiddles(tws_dst + 32 * mg + (m & 3), b.tw, g, w);
     radix16_fwd(v, w, p);
     if (4 * mg + tq < M) {
       uint32_t *dst = jb.dst + (static_cast<size_t>(jb.dst_row[m]) << 16) + col;
@@ -155,8 +186,13 @@ __global__ void __launch_bounds__(32 * kColWarps, MINB) k_modswitch_cols(const _
 
 void launch_modswitch_cols(const MSColBatch &b, int log_n, cudaStream_t s) {
   if (b.count <= 0 || log_n != 16) return;
-  int max_k = 0;
-  for (int j = 0; j < b.count; j++) max_k = b.jobs[j].K > max_k ? b.jobs[j].K : max_k;
+  int max_k = 0, max_m = 0;
+  for (int j = 0; j < b.count; j++) {
+    max_k = b.jobs[j].K > max_k ? b.jobs[j].K : max_k;
+    max_m = b.jobs[j].M > max_m ? b.jobs[j].M : max_m;
+  }
+  // twiddles: 128 bytes per prime of every group of four sources and targets
+  const size_t smem = max_k <= 4 ? 0 : 512 * static_cast<size_t>((max_k + 3) / 4 + (max_m + 3) / 4);
   // one CTA per 32 columns of a job, each converting all of the job's targets:
   // sharing a job's targets out over 2 to 6 CTAs (each repeating the source
   // stages) was slower at every size, down to the two one-source jobs of a
@@ -165,13 +201,13 @@ void launch_modswitch_cols(const MSColBatch &b, int log_n, cudaStream_t s) {
   // one, two and three parts)
   const dim3 grid(kRowLen / kCtaCols, b.count);
   if (max_k <= 4)
-    k_modswitch_cols<1, 7><<<grid, 32 * kColWarps, 0, s>>>(b);
+    k_modswitch_cols<1, 7><<<grid, 32 * kColWarps, smem, s>>>(b);
   else if (max_k <= 8)
-    k_modswitch_cols<2, 6><<<grid, 32 * kColWarps, 0, s>>>(b);
+    k_modswitch_cols<2, 6><<<grid, 32 * kColWarps, smem, s>>>(b);
   else if (max_k <= 12)
-    k_modswitch_cols<3, 5><<<grid, 32 * kColWarps, 0, s>>>(b);
+    k_modswitch_cols<3, 5><<<grid, 32 * kColWarps, smem, s>>>(b);
   else
-    k_modswitch_cols<4, 4><<<grid, 32 * kColWarps, 0, s>>>(b);
+    k_modswitch_cols<4, 4><<<grid, 32 * kColWarps, smem, s>>>(b);
 }
 
 }  // namespace chd

@@ -51,56 +51,98 @@ __global__ void __launch_bounds__(kColThreads) k_fwd_cols16(const __grid_constan
 
 // Row phase of the forward transform (input lazy from the column phase),
 // canonical output, with the optional ModDown epilogue (src2 * c1 - x) * c2.
-__global__ void __launch_bounds__(kRowThreads, 3) k_fwd_rows16(const __grid_constant__ RowBatch rb) {
-  __shared__ __align__(16) uint32_t sm[kRowLen];
-  const RowDesc &rd = rb.rows[blockIdx.y];
-  const uint32_t q = rd.q;
+// A CTA takes one row of one or (P = 2) two limbs of a prime.
+template <int P, int MINB>
+__global__ void __launch_bounds__(kRowThreads, MINB) k_fwd_rows16(const __grid_constant__ RowBatch rb) {
+  __shared__ __align__(16) uint32_t sm[P][kRowBuf];
+  const int first = P == 1 ? blockIdx.y : rb.first[blockIdx.y];
+  const bool two = P > 1 && rb.first[blockIdx.y + 1] - first > 1;
+  const uint32_t q = rb.rows[first].q;
   const int t = threadIdx.x, r = blockIdx.x;
-  const uint32_t *src = rd.dst + r * kRowLen;  // the column phase wrote dst
-  uint32_t x[16];
+  uint32_t x[P][16];
+  uint32_t *bufs[P];
 #pragma unroll
-  for (int k = 0; k < 16; k++) x[k] = src[t + 256 * k];
-  row_fwd(x, sm, rd.tw, r, t, q);
-  const int base = r * kRowLen + chunk_off(t);
+  for (int p = 0; p < P; p++) {
+    bufs[p] = sm[p];
+    if (p == 0 || two) {
+      const uint32_t *src = rb.rows[first + p].dst + r * kRowLen;  // the column phase wrote dst
 #pragma unroll
-  for (int k = 0; k < 16; k++) x[k] = reduce2q(x[k], q);
-  if (rd.flags & kModDownEpi) {
-    uint32_t v[16];
-    if (rd.flags & kHasSrc2) {
-      ld_chunks(rd.src2 + base, v);
-      if (rd.flags & kPadSrc2) {
-#pragma unroll
-        for (int k = 0; k < 16; k++) v[k] = reduce2q(shoup_lazy(v[k], rd.c1, rd.c1s, q), q);
-      }
-    } else {
-#pragma unroll
-      for (int k = 0; k < 16; k++) v[k] = 0;
+      for (int k = 0; k < 16; k++) x[p][k] = src[t + 256 * k];
     }
-#pragma unroll
-    for (int k = 0; k < 16; k++) x[k] = reduce2q(shoup_lazy(v[k] - x[k] + q, rd.c2, rd.c2s, q), q);
   }
-  st_chunks(rd.dst + base, x);
+  row_fwd_group<P>(x, two, bufs, rb.rows[first].tw, r, t, q);
+#pragma unroll
+  for (int p = 0; p < P; p++)
+    if (p == 0 || two) {
+#pragma unroll
+      for (int k = 0; k < 16; k++) x[p][k] = reduce2q(x[p][k], q);
+      group_st(bufs[p], t, x[p]);
+    }
+  __syncwarp();
+  const unsigned base = r * kRowLen + chunk_off(t);
+#pragma unroll
+  for (int p = 0; p < P; p++)
+    if (p == 0 || two) {
+      const RowDesc &rd = rb.rows[first + p];
+      uint32_t y[16];
+      chunk_ld(bufs[p], t, y);
+      if (rd.flags & kModDownEpi) {
+        uint32_t v[16];
+        if (rd.flags & kHasSrc2) {
+          ld_chunks(rd.src2 + base, v);
+          if (rd.flags & kPadSrc2) {
+#pragma unroll
+            for (int k = 0; k < 16; k++) v[k] = reduce2q(shoup_lazy(v[k], rd.c1, rd.c1s, q), q);
+          }
+        } else {
+#pragma unroll
+          for (int k = 0; k < 16; k++) v[k] = 0;
+        }
+#pragma unroll
+        for (int k = 0; k < 16; k++) y[k] = reduce2q(shoup_lazy(v[k] - y[k] + q, rd.c2, rd.c2s, q), q);
+      }
+      st_chunks(rd.dst + base, y);
+    }
 }
 
 // Inverse, row phase: Gentleman-Sande stages m = 32768 .. 16 (lazy output).
-__global__ void __launch_bounds__(kRowThreads, 3) k_inv_rows16(const __grid_constant__ RowBatch rb) {
-  __shared__ __align__(16) uint32_t sm[kRowLen];
-  const RowDesc &rd = rb.rows[blockIdx.y];
-  const uint32_t q = rd.q;
+template <int P, int MINB>
+__global__ void __launch_bounds__(kRowThreads, MINB) k_inv_rows16(const __grid_constant__ RowBatch rb) {
+  __shared__ __align__(16) uint32_t sm[P][kRowBuf];
+  const int first = P == 1 ? blockIdx.y : rb.first[blockIdx.y];
+  const bool two = P > 1 && rb.first[blockIdx.y + 1] - first > 1;
+  const uint32_t q = rb.rows[first].q;
   const int t = threadIdx.x, r = blockIdx.x;
-  const int base = r * kRowLen + chunk_off(t);
-  uint32_t x[16];
-  ld_chunks(rd.src + base, x);
-  if (rd.flags & kMulSrc2) {
-    uint32_t y[16];
-    ld_chunks(rd.src2 + base, y);
+  const unsigned base = r * kRowLen + chunk_off(t);
+  uint32_t x[P][16];
+  uint32_t *bufs[P];
 #pragma unroll
-    for (int k = 0; k < 16; k++) x[k] = mont_mul(x[k], y[k], q, rd.qinv);
+  for (int p = 0; p < P; p++) {
+    bufs[p] = sm[p];
+    if (p == 0 || two) ld_chunks(rb.rows[first + p].src + base, x[p]);
   }
-  row_inv(x, sm, rd.tw, r, t, q);
-  uint32_t *dst = rd.dst + r * kRowLen;
 #pragma unroll
-  for (int k = 0; k < 16; k++) dst[t + 256 * k] = x[k];
+  for (int p = 0; p < P; p++)
+    if (p == 0 || two) {
+      const RowDesc &rd = rb.rows[first + p];
+      if (rd.flags & kMulSrc2) {
+        uint32_t y[16];
+        ld_chunks(rd.src2 + base, y);
+#pragma unroll
+        for (int k = 0; k < 16; k++) x[p][k] = mont_mul(x[p][k], y[k], q, rd.qinv);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        chunk_st4(bufs[p], t, i, make_uint4(x[p][4 * i], x[p][4 * i + 1], x[p][4 * i + 2], x[p][4 * i + 3]));
+    }
+  row_inv_stored<P>(x, two, bufs, rb.rows[first].tw, r, t, q);
+#pragma unroll
+  for (int p = 0; p < P; p++)
+    if (p == 0 || two) {
+      uint32_t *dst = rb.rows[first + p].dst + r * kRowLen;
+#pragma unroll
+      for (int k = 0; k < 16; k++) dst[t + 256 * k] = x[p][k];
+    }
 }
 
 // Inverse, column phase: stages m = 8 .. 1, then x * c0, canonical or centred.
@@ -184,12 +226,36 @@ void launch_ntt_fwd_cols(const RowBatch &rb, int log_n, cudaStream_t s) {
   k_fwd_cols16<<<dim3(kRowLen / kColThreads, rb.count), kColThreads, 0, s>>>(rb);
 }
 
-void launch_ntt_fwd_rows(const RowBatch &rb, int log_n, cudaStream_t s) {
+namespace {
+// Neighbouring limbs of one prime share a CTA: rb.first receives the first
+// limb of each group of one or two; returns the number of groups.  Pairs of
+// rows run at 3 CTAs per SM (80 registers), single rows at 4 (64): pairs read
+// half the twiddles (raw transforms of 32 polynomials of 24 primes 377 us
+// against 387), but half as many CTAs leave SMs idle in small launches (one
+// multiplication at level 22, 23 pairs: 102.8 us against 100.7), so pairs are
+// taken from two waves of them on.
+constexpr int kPairWaves = 2 * 3 * 148;
+int pair_rows(RowBatch &rb) {
+  int groups = 0;
+  for (int i = 0; i < rb.count; groups++) {
+    rb.first[groups] = static_cast<uint16_t>(i);
+    i += i + 1 < rb.count && rb.rows[i + 1].tw == rb.rows[i].tw ? 2 : 1;
+  }
+  rb.first[groups] = static_cast<uint16_t>(rb.count);
+  return groups;
+}
+}  // namespace
+
+void launch_ntt_fwd_rows(RowBatch &rb, int log_n, cudaStream_t s) {
   if (rb.count <= 0) return;
-  k_fwd_rows16<<<dim3(kLimbRows, rb.count), kRowThreads, 0, s>>>(rb);
+  const int groups = pair_rows(rb);
+  if (groups == rb.count || groups * kLimbRows < kPairWaves)
+    k_fwd_rows16<1, 4><<<dim3(kLimbRows, rb.count), kRowThreads, 0, s>>>(rb);
+  else
+    k_fwd_rows16<2, 3><<<dim3(kLimbRows, groups), kRowThreads, 0, s>>>(rb);
 }
 
-void launch_ntt_fwd(const RowBatch &rb, int log_n, cudaStream_t s) {
+void launch_ntt_fwd(RowBatch &rb, int log_n, cudaStream_t s) {
   if (rb.count <= 0) return;
   if (log_n == 16) {
     launch_ntt_fwd_cols(rb, log_n, s);
@@ -201,15 +267,19 @@ void launch_ntt_fwd(const RowBatch &rb, int log_n, cudaStream_t s) {
   }
 }
 
-void launch_ntt_inv_rows(const RowBatch &rb, int log_n, cudaStream_t s) {
+void launch_ntt_inv_rows(RowBatch &rb, int log_n, cudaStream_t s) {
   if (rb.count <= 0) return;
-  k_inv_rows16<<<dim3(kLimbRows, rb.count), kRowThreads, 0, s>>>(rb);
+  const int groups = pair_rows(rb);
+  if (groups == rb.count || groups * kLimbRows < kPairWaves)
+    k_inv_rows16<1, 4><<<dim3(kLimbRows, rb.count), kRowThreads, 0, s>>>(rb);
+  else
+    k_inv_rows16<2, 3><<<dim3(kLimbRows, groups), kRowThreads, 0, s>>>(rb);
 }
 
-void launch_ntt_inv(const RowBatch &rb, int log_n, cudaStream_t s) {
+void launch_ntt_inv(RowBatch &rb, int log_n, cudaStream_t s) {
   if (rb.count <= 0) return;
   if (log_n == 16) {
-    k_inv_rows16<<<dim3(kLimbRows, rb.count), kRowThreads, 0, s>>>(rb);
+    launch_ntt_inv_rows(rb, log_n, s);
     k_inv_cols16<<<dim3(kRowLen / kColThreads, rb.count), kColThreads, 0, s>>>(rb);
   } else {
     size_t smem = sizeof(uint32_t) << log_n;
