@@ -17,6 +17,7 @@
 
 #include "arith.cuh"
 #include "kernels.h"
+#include "launch.cuh"
 
 namespace chd {
 namespace {
@@ -28,6 +29,7 @@ __global__ void k_modup_to_max(const __grid_constant__ ModUpToMaxDesc d) {
   const size_t n = static_cast<size_t>(d.n);
   const uint32_t *src = d.src[part];
   uint32_t *dst = d.dst[part] + static_cast<size_t>(r) * n;
+  grid_wait();
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<size_t>(gridDim.x) * blockDim.x) {
     if (d.nbase == 1) {
@@ -159,6 +161,7 @@ __global__ void __launch_bounds__(256) k_const_accum(const __grid_constant__ Con
   const size_t n = static_cast<size_t>(d.n);
   const size_t i = (static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
   if (i >= n) return;
+  grid_wait();
   uint32_t s[4] = {0, 0, 0, 0};
   for (int t = 0; t < d.terms; t++) {
     const uint32_t *src = d.src[t][part];
@@ -176,7 +179,7 @@ __global__ void __launch_bounds__(256) k_const_accum(const __grid_constant__ Con
 
 void launch_modup_to_max(const ModUpToMaxDesc &d, cudaStream_t s) {
   if (d.rows <= 0 || d.parts <= 0) return;
-  k_modup_to_max<<<dim3(64, d.rows, d.parts), 256, 0, s>>>(d);
+  launch_dependent(k_modup_to_max, dim3(64, d.rows, d.parts), 256, 0, s, d);
 }
 
 namespace {
@@ -270,7 +273,7 @@ void launch_pt_accum(const PtAccumDesc &d, cudaStream_t s, bool tune) {
 
 void launch_const_accum(const ConstAccumDesc &d, cudaStream_t s) {
   if (d.rows <= 0 || d.parts <= 0 || d.parts > kMaxConstAccumOuts || d.terms <= 0) return;
-  k_const_accum<<<dim3((d.n / 4 + 255) / 256, d.rows, d.parts), 256, 0, s>>>(d);
+  launch_dependent(k_const_accum, dim3((d.n / 4 + 255) / 256, d.rows, d.parts), 256, 0, s, d);
 }
 
 }  // namespace chd

@@ -8,11 +8,14 @@
 
 #include "arith.cuh"
 #include "kernels.h"
+#include "launch.cuh"
 
 namespace chd {
 namespace {
 
-__device__ __forceinline__ uint4 ld4(const uint32_t *p) { return __ldg(reinterpret_cast<const uint4 *>(p)); }
+// ld4c only in kernels that are not launched dependently (launch.cuh)
+__device__ __forceinline__ uint4 ld4(const uint32_t *p) { return *reinterpret_cast<const uint4 *>(p); }
+__device__ __forceinline__ uint4 ld4c(const uint32_t *p) { return __ldg(reinterpret_cast<const uint4 *>(p)); }
 __device__ __forceinline__ void st4(uint32_t *p, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   *reinterpret_cast<uint4 *>(p) = make_uint4(a, b, c, d);
 }
@@ -92,12 +95,12 @@ __global__ void __launch_bounds__(256) k_key_mac(const __grid_constant__ KeyMacD
   int i = 0;
   for (; i + 1 < d.beta; i += 2) {  // two digits per Montgomery reduction
     uint32_t mu0[4], kb0[4], ka0[4], mu1[4], kb1[4], ka1[4];
-    unpack(ld4(c.mu[i] + off), mu0);
-    unpack(ld4(d.kb[i] + koff), kb0);
-    unpack(ld4(d.ka[i] + koff), ka0);
-    unpack(ld4(c.mu[i + 1] + off), mu1);
-    unpack(ld4(d.kb[i + 1] + koff), kb1);
-    unpack(ld4(d.ka[i + 1] + koff), ka1);
+    unpack(ld4c(c.mu[i] + off), mu0);
+    unpack(ld4c(d.kb[i] + koff), kb0);
+    unpack(ld4c(d.ka[i] + koff), ka0);
+    unpack(ld4c(c.mu[i + 1] + off), mu1);
+    unpack(ld4c(d.kb[i + 1] + koff), kb1);
+    unpack(ld4c(d.ka[i + 1] + koff), ka1);
 #pragma unroll
     for (int l = 0; l < 4; l++) {
       sb[l] = add_mod(sb[l], mont_mac2(mu0[l], kb0[l], mu1[l], kb1[l], q, qn), q);
@@ -106,9 +109,9 @@ __global__ void __launch_bounds__(256) k_key_mac(const __grid_constant__ KeyMacD
   }
   if (i < d.beta) {
     uint32_t mu[4], kb[4], ka[4];
-    unpack(ld4(c.mu[i] + off), mu);
-    unpack(ld4(d.kb[i] + koff), kb);
-    unpack(ld4(d.ka[i] + koff), ka);
+    unpack(ld4c(c.mu[i] + off), mu);
+    unpack(ld4c(d.kb[i] + koff), kb);
+    unpack(ld4c(d.ka[i] + koff), ka);
 #pragma unroll
     for (int l = 0; l < 4; l++) {
       sb[l] = add_mod(sb[l], mont_mul(mu[l], kb[l], q, qi), q);
@@ -119,13 +122,13 @@ __global__ void __launch_bounds__(256) k_key_mac(const __grid_constant__ KeyMacD
     const uint32_t pp = d.p_prod[r];
     if (c.d0) {
       uint32_t v[4];
-      unpack(ld4(c.d0 + off), v);
+      unpack(ld4c(c.d0 + off), v);
 #pragma unroll
       for (int l = 0; l < 4; l++) sb[l] = add_mod(sb[l], mont_mul(v[l], pp, q, qi), q);
     }
     if (c.d1) {
       uint32_t v[4];
-      unpack(ld4(c.d1 + off), v);
+      unpack(ld4c(c.d1 + off), v);
 #pragma unroll
       for (int l = 0; l < 4; l++) sa[l] = add_mod(sa[l], mont_mul(v[l], pp, q, qi), q);
     }
@@ -141,6 +144,7 @@ __global__ void __launch_bounds__(256) k_elem(const __grid_constant__ ElemBatch 
   const ElemRow &e = eb.rows[blockIdx.y];
   const int i0 = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (i0 >= n) return;
+  grid_wait();
   const uint32_t q = e.q;
   const int32_t qi = e.qinv;
   uint32_t a[4], b[4], c[4], o[4];
@@ -178,6 +182,7 @@ __global__ void __launch_bounds__(256) k_tensor(const __grid_constant__ TensorBa
   const TensorRow &t = tb.rows[blockIdx.y];
   const int i0 = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (i0 >= n) return;
+  grid_wait();
   const uint32_t q = t.q;
   const int32_t qi = t.qinv;
   uint32_t b1[4], a1[4], b2[4], a2[4], o0[4], o1[4], o2[4];
@@ -214,6 +219,7 @@ __global__ void __launch_bounds__(256) k_permute(const __grid_constant__ Permute
   const PermuteRow &p = pb.rows[blockIdx.y];
   const int k0 = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (k0 >= n) return;
+  grid_wait();
   uint32_t slot[4];
 #pragma unroll
   for (int l = 0; l < 4; l++) slot[l] = galois_src(k0 + l, pb.galois, log_n);
@@ -267,9 +273,9 @@ __global__ void __launch_bounds__(256, MINB) k_hoisted(const __grid_constant__ H
   uint32_t mu[BMAX][4];
 #pragma unroll
   for (int i = 0; i < BMAX; i++)
-    if (i < d.beta) unpack(ld4(d.mu[c][i] + off), mu[i]);
+    if (i < d.beta) unpack(ld4c(d.mu[c][i] + off), mu[i]);
   uint32_t bxp[4] = {0, 0, 0, 0};
-  if (r < d.nq) unpack(ld4(d.bxp[c] + off), bxp);
+  if (r < d.nq) unpack(ld4c(d.bxp[c] + off), bxp);
   for (int j = 0; j < d.R; j++) {
     uint32_t sb[4], sa[4] = {0, 0, 0, 0};
 #pragma unroll
@@ -278,10 +284,10 @@ __global__ void __launch_bounds__(256, MINB) k_hoisted(const __grid_constant__ H
     for (int i = 0; i < BMAX; i += 2) {
       if (i + 1 < d.beta) {  // two digits per Montgomery reduction
         uint32_t kb0[4], ka0[4], kb1[4], ka1[4];
-        unpack(ld4(d.kb[j][i] + koff), kb0);
-        unpack(ld4(d.ka[j][i] + koff), ka0);
-        unpack(ld4(d.kb[j][i + 1] + koff), kb1);
-        unpack(ld4(d.ka[j][i + 1] + koff), ka1);
+        unpack(ld4c(d.kb[j][i] + koff), kb0);
+        unpack(ld4c(d.ka[j][i] + koff), ka0);
+        unpack(ld4c(d.kb[j][i + 1] + koff), kb1);
+        unpack(ld4c(d.ka[j][i + 1] + koff), ka1);
 #pragma unroll
         for (int l = 0; l < 4; l++) {
           sb[l] = add_mod(sb[l], mont_mac2(mu[i][l], kb0[l], mu[i + 1][l], kb1[l], q, qn), q);
@@ -289,8 +295,8 @@ __global__ void __launch_bounds__(256, MINB) k_hoisted(const __grid_constant__ H
         }
       } else if (i < d.beta) {
         uint32_t kb[4], ka[4];
-        unpack(ld4(d.kb[j][i] + koff), kb);
-        unpack(ld4(d.ka[j][i] + koff), ka);
+        unpack(ld4c(d.kb[j][i] + koff), kb);
+        unpack(ld4c(d.ka[j][i] + koff), ka);
 #pragma unroll
         for (int l = 0; l < 4; l++) {
           sb[l] = add_mod(sb[l], mont_mul(mu[i][l], kb[l], q, qi), q);
@@ -347,7 +353,7 @@ void launch_elementwise(ElemOp op, const ElemBatch &b, int log_n, cudaStream_t s
   dim3 grid((n / 4 + 255) / 256, b.count);
   switch (op) {
 #define CHD_CASE(OP) \
-  case OP: k_elem<OP><<<grid, 256, 0, s>>>(b, log_n); break;
+  case OP: launch_dependent(k_elem<OP>, grid, 256, 0, s, b, log_n); break;
     CHD_CASE(ElemOp::kAdd)
     CHD_CASE(ElemOp::kSub)
     CHD_CASE(ElemOp::kNeg)
@@ -367,13 +373,13 @@ void launch_elementwise(ElemOp op, const ElemBatch &b, int log_n, cudaStream_t s
 void launch_tensor(const TensorBatch &b, int log_n, cudaStream_t s) {
   if (b.count <= 0) return;
   const int n = 1 << log_n;
-  k_tensor<<<dim3((n / 4 + 255) / 256, b.count), 256, 0, s>>>(b, log_n);
+  launch_dependent(k_tensor, dim3((n / 4 + 255) / 256, b.count), 256, 0, s, b, log_n);
 }
 
 void launch_permute(const PermuteBatch &b, int log_n, cudaStream_t s) {
   if (b.count <= 0) return;
   const int n = 1 << log_n;
-  k_permute<<<dim3((n / 4 + 255) / 256, b.count), 256, 0, s>>>(b, log_n);
+  launch_dependent(k_permute, dim3((n / 4 + 255) / 256, b.count), 256, 0, s, b, log_n);
 }
 
 namespace {

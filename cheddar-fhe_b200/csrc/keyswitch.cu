@@ -18,6 +18,7 @@
 // ModDown column pass).
 #include "arith.cuh"
 #include "kernels.h"
+#include "launch.cuh"
 #include "ntt_common.cuh"
 
 namespace chd {
@@ -60,7 +61,7 @@ __device__ __forceinline__ void inner_product(const KSRowsCt &c, const KSRowsLev
 #pragma unroll 1
   for (int e = 0; e < 4; e++) {
     auto ld4 = [&](const uint32_t *p, uint32_t *x) {
-      const uint4 v4 = __ldg(reinterpret_cast<const uint4 *>(p + 64 * e));
+      const uint4 v4 = *reinterpret_cast<const uint4 *>(p + 64 * e);
       x[0] = v4.x; x[1] = v4.y; x[2] = v4.z; x[3] = v4.w;
     };
     uint64_t sb[4] = {0, 0, 0, 0}, sa[4] = {0, 0, 0, 0};
@@ -160,6 +161,7 @@ __global__ void __launch_bounds__(kRowThreads, 4) k_ks_rows(const __grid_constan
   const int t = threadIdx.x, r = blockIdx.y;
   const size_t row = static_cast<size_t>(j) * 65536 + r * kRowLen;
   const int own = L.own_digit[j], beta = L.beta;
+  grid_wait();
   // ---- ModUp NTT rows: each digit's row stays in its buffer
   for (int i = 0; i < beta; i++) {
     if (own == i) continue;
@@ -207,7 +209,7 @@ void launch_ks_rows(const KSRowsDesc &d, int log_n, cudaStream_t s) {
   int bufs = 2;
   for (int i = 0; i < d.nlv; i++) bufs = d.lv[i].beta > bufs ? d.lv[i].beta : bufs;
   cudaFuncSetAttribute(k_ks_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDigits * kRowBuf * 4);
-  k_ks_rows<<<dim3(d.count, kLimbRows, d.max_rows), kRowThreads, bufs * kRowBuf * 4, s>>>(d);
+  launch_dependent(k_ks_rows, dim3(d.count, kLimbRows, d.max_rows), kRowThreads, bufs * kRowBuf * 4, s, d);
 }
 
 }  // namespace chd

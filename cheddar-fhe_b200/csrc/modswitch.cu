@@ -40,6 +40,7 @@
 // never wait for one another.
 #include "arith.cuh"
 #include "kernels.h"
+#include "launch.cuh"
 #include "ntt_common.cuh"
 
 namespace chd {
@@ -84,30 +85,33 @@ __global__ void __launch_bounds__(32 * kColWarps, MINB) k_modswitch_cols(const _
   const int lane = threadIdx.x & 31, tq = lane & 3;
   const int col = (blockIdx.x * kColWarps + (threadIdx.x >> 5)) * 8 + (lane >> 2);
   const int K = jb.K, M = jb.M;
-  // The fifteen twiddles of every source and target prime (the column stages
-  // use the first sixteen table entries): [group of four primes][pair of
-  // entries][prime], so that the four primes of a warp's 16-byte access lie
-  // in 64 contiguous bytes.  Read from the tables by every warp they cost
-  // four cache lines per access, and the pass filled the cache's data path
-  // (76 % of its peak; ModUp 88 -> 85 us, ModDown 70.5 -> 68).  With up to
-  // four sources there is too little work for the detour (a plaintext product
-  // and rescale at level 5: 24.0 us from the tables, 25.8 us staged).
-  constexpr bool kStaged = KR > 1;
+  const int steps = (K + 7) / 8;  // K steps of 8 sources in the fragment table
+  const int groups = (M + 3) / 4;
+  // Staged in shared memory, before the wait for the kernel in front: what
+  // every warp of the CTA would otherwise fetch for itself, at four cache
+  // lines per access (the lanes of a quad need four different primes) and in
+  // chains of dependent loads.
+  //   tws, tws_dst: the fifteen twiddles of every source and target prime (the
+  //     column stages use the first sixteen table entries), [group of four
+  //     primes][pair of entries][prime], 64 contiguous bytes per access;
+  //   prm: prime, inverse and destination row of every target;
+  //   frg: the B fragments.
   extern __shared__ uint4 tws[];
-  uint4 *tws_dst = tws + 32 * KR;
-  for (int i = threadIdx.x; i < (kStaged ? 8 * (K + M) : 0); i += 32 * kColWarps) {
+  uint4 *const tws_dst = tws + 32 * KR, *const prm = tws_dst + 32 * groups, *const frg = prm + 4 * groups;
+  for (int i = threadIdx.x; i < 8 * (K + M); i += 32 * kColWarps) {
     const int k = i >> 3, c = i & 7;
     const bool src = k < K;
     const int g = src ? jb.src_gidx[k] : jb.dst_gidx[k - K], x = src ? k : k - K;
     const uint2 *tab = (src ? b.itw : b.tw) + (static_cast<size_t>(g) << 16);
     (src ? tws : tws_dst)[32 * (x >> 2) + 4 * c + (x & 3)] = __ldg(reinterpret_cast<const uint4 *>(tab) + c);
   }
-  if (kStaged) __syncthreads();
-  auto twiddles = [&](const uint4 *p, const uint2 *table, int g, uint2 *w) {
-    if (!kStaged) {
-      tw_radix16(table + (static_cast<size_t>(g) << 16), 1, w);
-      return;
-    }
+  for (int m = threadIdx.x; m < M; m += 32 * kColWarps) {
+    const int g = jb.dst_gidx[m];
+    prm[m] = make_uint4(__ldg(b.primes + g), static_cast<uint32_t>(__ldg(b.qinvs + g)), jb.dst_row[m], 0);
+  }
+  for (int i = threadIdx.x; i < 32 * groups * (steps + 1); i += 32 * kColWarps) frg[i] = __ldg(jb.frag + i);
+  grid_wait();
+  auto twiddles = [&](const uint4 *p, uint2 *w) {
 #pragma unroll
     for (int c = 0; c < 8; c++) {
       const uint4 v = p[4 * c];
@@ -128,8 +132,9 @@ __global__ void __launch_bounds__(32 * kColWarps, MINB) k_modswitch_cols(const _
       const uint32_t c0 = jb.c0[k], c0s = jb.c0s[k];
       uint2 w[16];
 #pragma unroll
-      for (int e = 0; e < 16; e++) xs[i][e] = __ldg(src + e * kRowLen);
-      twiddles(tws + 32 * i + (k & 3), b.itw, g, w);
+      for (int e = 0; e < 16; e++) xs[i][e] = src[e * kRowLen];
+      if (i == 0) __syncthreads();  // the staged tables
+      twiddles(tws + 32 * i + (k & 3), w);
       radix16_inv(xs[i], w, q);
 #pragma unroll
       for (int e = 0; e < 16; e++)
@@ -141,18 +146,16 @@ __global__ void __launch_bounds__(32 * kColWarps, MINB) k_modswitch_cols(const _
   }
   // ---- four targets at a time: MMAs, reduction, NTT column stages, store
   constexpr int kSteps = (KR + 1) / 2;
-  const int steps = (K + 7) / 8;  // K steps of 8 sources in the fragment table
-  const int groups = (M + 3) / 4;
   for (int mg = 0; mg < groups; mg++) {
-    const uint4 *frag = jb.frag + static_cast<size_t>(mg) * (steps + 1) * 32 + lane;
+    const uint4 *frag = frg + mg * (steps + 1) * 32 + lane;
     const int m = min(4 * mg + tq, M - 1);
-    const int g = jb.dst_gidx[m];
-    const uint32_t p = __ldg(b.primes + g);
-    const int32_t pinv = __ldg(b.qinvs + g);
+    const uint4 pr = prm[m];
+    const uint32_t p = pr.x;
+    const int32_t pinv = static_cast<int32_t>(pr.y);
     uint4 bw[kSteps];
 #pragma unroll
-    for (int s = 0; s < kSteps; s++) bw[s] = s < steps ? __ldg(frag + 32 * s) : make_uint4(0, 0, 0, 0);
-    const uint4 cc = __ldg(frag + 32 * steps);
+    for (int s = 0; s < kSteps; s++) bw[s] = s < steps ? frag[32 * s] : make_uint4(0, 0, 0, 0);
+    const uint4 cc = frag[32 * steps];
     uint32_t v[16];
 #pragma unroll
     for (int e = 0; e < 16; e += 2) {
@@ -172,10 +175,10 @@ __global__ void __launch_bounds__(32 * kColWarps, MINB) k_modswitch_cols(const _
       v[e + 1] = join(lo[2], lo[3], hi[2], hi[3], p, pinv);
     }
     uint2 w[16];
-    twiddles(tws_dst + 32 * mg + (m & 3), b.tw, g, w);
+    twiddles(tws_dst + 32 * mg + (m & 3), w);
     radix16_fwd(v, w, p);
     if (4 * mg + tq < M) {
-      uint32_t *dst = jb.dst + (static_cast<size_t>(jb.dst_row[m]) << 16) + col;
+      uint32_t *dst = jb.dst + (static_cast<size_t>(pr.z) << 16) + col;
 #pragma unroll
       for (int e = 0; e < 16; e++) dst[e * kRowLen] = v[e];
     }
@@ -191,8 +194,10 @@ void launch_modswitch_cols(const MSColBatch &b, int log_n, cudaStream_t s) {
     max_k = b.jobs[j].K > max_k ? b.jobs[j].K : max_k;
     max_m = b.jobs[j].M > max_m ? b.jobs[j].M : max_m;
   }
-  // twiddles: 128 bytes per prime of every group of four sources and targets
-  const size_t smem = max_k <= 4 ? 0 : 512 * static_cast<size_t>((max_k + 3) / 4 + (max_m + 3) / 4);
+  // the kernel's staged tables: 512 bytes of twiddles per group of four
+  // primes, 64 of prime data and 512 per fragment step and group of targets
+  const int groups = (max_m + 3) / 4, steps = (max_k + 7) / 8;
+  const size_t smem = 512 * ((max_k + 3) / 4 + groups) + 64 * groups + 512 * static_cast<size_t>(groups) * (steps + 1);
   // one CTA per 32 columns of a job, each converting all of the job's targets:
   // sharing a job's targets out over 2 to 6 CTAs (each repeating the source
   // stages) was slower at every size, down to the two one-source jobs of a
@@ -200,14 +205,18 @@ void launch_modswitch_cols(const MSColBatch &b, int log_n, cudaStream_t s) {
   // 25.6 us in two; a multiplication at level 22: 98.7, 103.5 and 107.7 us in
   // one, two and three parts)
   const dim3 grid(kRowLen / kCtaCols, b.count);
+  auto go = [&](auto kern) {
+    // 35 KiB at most (16 sources, 64 targets)
+    launch_dependent(kern, grid, 32 * kColWarps, smem, s, b);
+  };
   if (max_k <= 4)
-    k_modswitch_cols<1, 7><<<grid, 32 * kColWarps, smem, s>>>(b);
+    go(k_modswitch_cols<1, 7>);
   else if (max_k <= 8)
-    k_modswitch_cols<2, 6><<<grid, 32 * kColWarps, smem, s>>>(b);
+    go(k_modswitch_cols<2, 6>);
   else if (max_k <= 12)
-    k_modswitch_cols<3, 5><<<grid, 32 * kColWarps, smem, s>>>(b);
+    go(k_modswitch_cols<3, 5>);
   else
-    k_modswitch_cols<4, 4><<<grid, 32 * kColWarps, smem, s>>>(b);
+    go(k_modswitch_cols<4, 4>);
 }
 
 }  // namespace chd

@@ -21,6 +21,7 @@
 // fits in shared memory and one kernel runs every stage.
 #include "arith.cuh"
 #include "kernels.h"
+#include "launch.cuh"
 #include "ntt_common.cuh"
 
 namespace chd {
@@ -37,9 +38,10 @@ __global__ void __launch_bounds__(kColThreads) k_fwd_cols16(const __grid_constan
   const int c = blockIdx.x * kColThreads + threadIdx.x;
   uint32_t x[16];
   uint2 w[16];
+  tw_radix16(rd.tw, 1, w);
+  grid_wait();
 #pragma unroll
   for (int k = 0; k < 16; k++) x[k] = rd.src[k * kRowLen + c];
-  tw_radix16(rd.tw, 1, w);
   if (rd.flags & kPreMult) {
 #pragma unroll
     for (int k = 0; k < 16; k++) x[k] = shoup_lazy(x[k], rd.c0, rd.c0s, q);
@@ -61,6 +63,7 @@ __global__ void __launch_bounds__(kRowThreads, MINB) k_fwd_rows16(const __grid_c
   const int t = threadIdx.x, r = blockIdx.x;
   uint32_t x[P][16];
   uint32_t *bufs[P];
+  grid_wait();
 #pragma unroll
   for (int p = 0; p < P; p++) {
     bufs[p] = sm[p];
@@ -116,6 +119,7 @@ __global__ void __launch_bounds__(kRowThreads, MINB) k_inv_rows16(const __grid_c
   const unsigned base = r * kRowLen + chunk_off(t);
   uint32_t x[P][16];
   uint32_t *bufs[P];
+  grid_wait();
 #pragma unroll
   for (int p = 0; p < P; p++) {
     bufs[p] = sm[p];
@@ -153,9 +157,10 @@ __global__ void __launch_bounds__(kColThreads) k_inv_cols16(const __grid_constan
   uint32_t *p = rd.dst;  // the row phase wrote dst
   uint32_t x[16];
   uint2 w[16];
+  tw_radix16(rd.tw, 1, w);
+  grid_wait();
 #pragma unroll
   for (int k = 0; k < 16; k++) x[k] = p[k * kRowLen + c];
-  tw_radix16(rd.tw, 1, w);
   radix16_inv(x, w, q);
   const bool centre_out = (rd.flags & kCentre) != 0;
 #pragma unroll
@@ -175,6 +180,7 @@ __global__ void __launch_bounds__(1024) k_small(const __grid_constant__ RowBatch
   const uint32_t q = rd.q;
   const uint2 *tw = rd.tw;
   const int n = 1 << log_n, half = n >> 1;
+  grid_wait();
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     uint32_t v = rd.src[i];
     if (kFwd && (rd.flags & kPreMult)) v = shoup_lazy(v, rd.c0, rd.c0s, q);
@@ -223,7 +229,7 @@ __global__ void __launch_bounds__(1024) k_small(const __grid_constant__ RowBatch
 
 void launch_ntt_fwd_cols(const RowBatch &rb, int log_n, cudaStream_t s) {
   if (rb.count <= 0) return;
-  k_fwd_cols16<<<dim3(kRowLen / kColThreads, rb.count), kColThreads, 0, s>>>(rb);
+  launch_dependent(k_fwd_cols16, dim3(kRowLen / kColThreads, rb.count), kColThreads, 0, s, rb);
 }
 
 namespace {
@@ -250,9 +256,9 @@ void launch_ntt_fwd_rows(RowBatch &rb, int log_n, cudaStream_t s) {
   if (rb.count <= 0) return;
   const int groups = pair_rows(rb);
   if (groups == rb.count || groups * kLimbRows < kPairWaves)
-    k_fwd_rows16<1, 4><<<dim3(kLimbRows, rb.count), kRowThreads, 0, s>>>(rb);
+    launch_dependent(k_fwd_rows16<1, 4>, dim3(kLimbRows, rb.count), kRowThreads, 0, s, rb);
   else
-    k_fwd_rows16<2, 3><<<dim3(kLimbRows, groups), kRowThreads, 0, s>>>(rb);
+    launch_dependent(k_fwd_rows16<2, 3>, dim3(kLimbRows, groups), kRowThreads, 0, s, rb);
 }
 
 void launch_ntt_fwd(RowBatch &rb, int log_n, cudaStream_t s) {
@@ -263,7 +269,7 @@ void launch_ntt_fwd(RowBatch &rb, int log_n, cudaStream_t s) {
   } else {
     size_t smem = sizeof(uint32_t) << log_n;
     cudaFuncSetAttribute(k_small<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024);
-    k_small<true><<<rb.count, 1024, smem, s>>>(rb, log_n);
+    launch_dependent(k_small<true>, rb.count, 1024, smem, s, rb, log_n);
   }
 }
 
@@ -271,20 +277,20 @@ void launch_ntt_inv_rows(RowBatch &rb, int log_n, cudaStream_t s) {
   if (rb.count <= 0) return;
   const int groups = pair_rows(rb);
   if (groups == rb.count || groups * kLimbRows < kPairWaves)
-    k_inv_rows16<1, 4><<<dim3(kLimbRows, rb.count), kRowThreads, 0, s>>>(rb);
+    launch_dependent(k_inv_rows16<1, 4>, dim3(kLimbRows, rb.count), kRowThreads, 0, s, rb);
   else
-    k_inv_rows16<2, 3><<<dim3(kLimbRows, groups), kRowThreads, 0, s>>>(rb);
+    launch_dependent(k_inv_rows16<2, 3>, dim3(kLimbRows, groups), kRowThreads, 0, s, rb);
 }
 
 void launch_ntt_inv(RowBatch &rb, int log_n, cudaStream_t s) {
   if (rb.count <= 0) return;
   if (log_n == 16) {
     launch_ntt_inv_rows(rb, log_n, s);
-    k_inv_cols16<<<dim3(kRowLen / kColThreads, rb.count), kColThreads, 0, s>>>(rb);
+    launch_dependent(k_inv_cols16, dim3(kRowLen / kColThreads, rb.count), kColThreads, 0, s, rb);
   } else {
     size_t smem = sizeof(uint32_t) << log_n;
     cudaFuncSetAttribute(k_small<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024);
-    k_small<false><<<rb.count, 1024, smem, s>>>(rb, log_n);
+    launch_dependent(k_small<false>, rb.count, 1024, smem, s, rb, log_n);
   }
 }
 

@@ -252,7 +252,7 @@ __device__ __forceinline__ void row_inv_stored(uint32_t (&x)[P][16], bool two, u
 __device__ __forceinline__ void ld_chunks(const uint32_t *p, uint32_t *x) {
 #pragma unroll
   for (int i = 0; i < 4; i++) {
-    const uint4 v = __ldg(reinterpret_cast<const uint4 *>(p + 64 * i));
+    const uint4 v = *reinterpret_cast<const uint4 *>(p + 64 * i);
     x[4 * i] = v.x; x[4 * i + 1] = v.y; x[4 * i + 2] = v.z; x[4 * i + 3] = v.w;
   }
 }
