@@ -474,6 +474,17 @@ void Context64::shoup(u64 c, int g, u64 *w, u64 *ws) const {
 
 void Context64::mont_shoup(u64 c, int g, u64 *w, u64 *ws) const { shoup(mul_mod(c, r_inv[g], P->primes[g]), g, w, ws); }
 
+// Table position of twiddle j (N = 2^16): its index, except that the 2, 4 and 8
+// pairs that a thread of the row phase needs for stages m = 8192, 16384 and
+// 32768 lie 256 apart within the row's pairs (TwLast, w64_kernels.cu), so that
+// a warp's loads are contiguous.
+static int tw_position64(int j) {
+  if (j < 8192) return j;
+  const int s = j < 16384 ? 1 : j < 32768 ? 2 : 3, base = 4096 << s, o = j - base;
+  const int row = o >> (8 + s), i = o & ((256 << s) - 1);
+  return base + (row << (8 + s)) + 256 * (i & ((1 << s) - 1)) + (i >> s);
+}
+
 Status Context64::init(const ParamSpec64 &spec, int dev, std::string *err) {
   P = Params64::create(spec, err);
   if (!P) return kErrInvalidArg;
@@ -491,6 +502,8 @@ Status Context64::init(const ParamSpec64 &spec, int dev, std::string *err) {
   mont_conv.resize(np_all);
   r_inv.resize(np_all);
   std::vector<u64> pw(n), pwi(n);
+  narrow = true;
+  for (u64 q : P->primes) narrow = narrow && q < (1ull << 58);
   for (int g = 0; g < np_all; g++) {
     const u64 q = P->primes[g];
     const u64 psi = primitive_root(2ull * n, q), psi_inv = inv_mod(psi, q);
@@ -507,8 +520,9 @@ Status Context64::init(const ParamSpec64 &spec, int dev, std::string *err) {
     for (int j = 0; j < n; j++) {
       const unsigned r = brev(j, P->log_n);
       auto sh = [q](u64 w) { return static_cast<u64>((static_cast<u128>(w) << 64) / q); };
-      tw[static_cast<size_t>(g) * n + j] = make_ulonglong2(pw[r], sh(pw[r]));
-      itw[static_cast<size_t>(g) * n + j] = make_ulonglong2(pwi[r], sh(pwi[r]));
+      const size_t o = static_cast<size_t>(g) * n + tw_position64(j);
+      tw[o] = make_ulonglong2(pw[r], sh(pw[r]));
+      itw[o] = make_ulonglong2(pwi[r], sh(pwi[r]));
     }
   }
   if (cudaMalloc(&d_primes, np_all * 8) != cudaSuccess || cudaMalloc(&d_qinv, np_all * 8) != cudaSuccess ||
@@ -632,6 +646,7 @@ Status Context64::modup(int level, const u64 *src, u64 *dst) {
   BConv64Batch b{};
   b.primes = d_primes;
   b.qinvs = d_qinv;
+  b.narrow = narrow;
   const size_t out_words = static_cast<size_t>(tot) * n;
   rows.clear();
   for (int i = 0; i < m.beta; i++) {
@@ -721,6 +736,7 @@ Status Context64::moddown(int level, MDType type, const u64 *const *src, u64 *co
   BConv64Batch b{};
   b.primes = d_primes;
   b.qinvs = d_qinv;
+  b.narrow = narrow;
   for (int p = 0; p < npoly; p++) {
     BConv64Job &j = b.jobs[b.count++];
     j.xt = xt + static_cast<size_t>(p) * src_len * n;

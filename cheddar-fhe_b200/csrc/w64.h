@@ -112,6 +112,7 @@ class Context64 {
   i64 *d_qinv = nullptr;
   ulonglong2 *d_tw = nullptr, *d_itw = nullptr;  // [nprimes][N] (w, floor(w 2^64 / q))
   std::vector<u64> n_inv, mont_conv, r_inv, n_inv_mont_inv;
+  bool narrow = false;  // every prime below 2^58 (k64_bconv)
   std::vector<u64> p_prod;  // Montgomery P mod q_i for the q primes of the key basis
   std::vector<std::unique_ptr<LevelMS64>> ms;  // index level + 1
   const LevelMS64 &lms(int level);
@@ -179,7 +180,7 @@ struct Row64 {
   uint32_t flags, pad_;
   u64 c0, c0s, c1, c1s, c2, c2s;
 };
-constexpr int kMaxRows64 = 64;
+constexpr int kMaxRows64 = 128;  // 13 KiB of launch parameters
 struct RowBatch64 {
   int count;
   Row64 rows[kMaxRows64];
@@ -200,6 +201,7 @@ struct BConv64Job {
 constexpr int kMaxBConv64Jobs = 16;
 struct BConv64Batch {
   int count;
+  bool narrow;  // every prime of the context is below 2^58
   const u64 *primes;
   const i64 *qinvs;
   BConv64Job jobs[kMaxBConv64Jobs];
