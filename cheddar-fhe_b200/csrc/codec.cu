@@ -19,6 +19,7 @@
 #include <complex>
 
 #include "host.h"
+#include "launch.cuh"
 #include "kernels.h"
 
 namespace chd {
@@ -36,36 +37,77 @@ __device__ __forceinline__ double2 cmul(double2 y, double2 t) {
                       __dadd_rn(__dmul_rn(y.x, t.y), __dmul_rn(y.y, t.x)));
 }
 
-// One stage of Encoder::SpecialIFFT (Encode.cpp:84-107): butterflies at
-// distance `stride`, twiddle index (st8 - (5^j mod 2N) mod st8) * gap
-__global__ void k_special_ifft_stage(double2 *d, int ns, int stride, const double2 *tw, const int *galois, int M) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= ns / 2) return;
-  const int j = b % stride, i = (b / stride) * 2 * stride;
-  const int st8 = stride << 3, gap = M / st8;
-  const int ti = (st8 - galois[j] % st8) * gap;
-  const double2 u = d[i + j], v = d[i + j + stride];
-  d[i + j] = dadd2(u, v);
-  d[i + j + stride] = cmul(dsub2(u, v), tw[ti]);
+// Stages of Encoder::SpecialIFFT (Encode.cpp:84-107; butterflies at distance
+// `stride`, twiddle index (st8 - (5^j mod 2N) mod st8) * gap, strides falling)
+// or Encoder::SpecialFFT (Encode.cpp:109-133; rising) whose strides lie in
+// [lo, lo 2^(nb-1)], run in shared memory: a CTA owns the 2^nb elements that
+// these stages connect, for 2^cb neighbouring columns.  Every butterfly does
+// the arithmetic of its own stage, so the doubles do not depend on how stages
+// are grouped.  BREV bit-reverses (BitReverseVector,
+// include/common/CommonUtils.h) on the way out of the inverse or into the
+// forward transform.
+//
+// One launch per stage cost 3.3 to 4.3 us each plus its gap, for 15 stages of
+// 2^15 slots; now two launches run them all.
+constexpr int kFftBits = 10;  // elements per CTA (log2), 16 KiB
+template <bool INV, bool BREV>
+__global__ void __launch_bounds__(512) k_special_stages(const double2 *src, double2 *dst, int lns, int llo, int nb, int cb,
+                                                        const double2 *tw, const int *galois, int M) {
+  __shared__ double2 sm[1 << kFftBits];
+  const int size = 1 << (nb + cb), lo = 1 << llo, cols = 1 << cb;
+  // element l of the tile: FFT index l >> cb, column l & (cols - 1)
+  const int tiles_per_block = lo >> cb;  // column tiles below one FFT block
+  const int blk = blockIdx.x / tiles_per_block, ct = blockIdx.x % tiles_per_block;
+  const int base = (blk << (llo + nb)) + (ct << cb);
+  auto at = [&](int l) { return base + ((l >> cb) << llo) + (l & (cols - 1)); };
+  auto rev = [&](int i) { return lns ? static_cast<int>(__brev(static_cast<unsigned>(i)) >> (32 - lns)) : 0; };
+  grid_wait();
+  for (int l = threadIdx.x; l < size; l += blockDim.x) sm[l] = src[!INV && BREV ? rev(at(l)) : at(l)];
+  __syncthreads();
+  for (int st = 0; st < nb; st++) {
+    const int ls = INV ? nb - 1 - st : st;  // FFT-index distance 2^ls, stride lo 2^ls
+    const int stride = lo << ls, st8 = stride << 3, gap = M / st8;
+    for (int h = threadIdx.x; h < size / 2; h += blockDim.x) {
+      const int f = h >> cb, c = h & (cols - 1);
+      const int f0 = ((f >> ls) << (ls + 1)) + (f & ((1 << ls) - 1));
+      const int l0 = (f0 << cb) + c, l1 = l0 + (1 << (ls + cb));
+      const int g = galois[at(l0) & (stride - 1)] % st8;
+      if (INV) {
+        const double2 u = sm[l0], v = sm[l1];
+        sm[l0] = dadd2(u, v);
+        sm[l1] = cmul(dsub2(u, v), tw[(st8 - g) * gap]);
+      } else {
+        const double2 x = sm[l0], y = cmul(sm[l1], tw[g * gap]);
+        sm[l0] = dadd2(x, y);
+        sm[l1] = dsub2(x, y);
+      }
+    }
+    __syncthreads();
+  }
+  for (int l = threadIdx.x; l < size; l += blockDim.x) dst[INV && BREV ? rev(at(l)) : at(l)] = sm[l];
 }
 
-// One stage of Encoder::SpecialFFT (Encode.cpp:109-133)
-__global__ void k_special_fft_stage(double2 *d, int ns, int stride, const double2 *tw, const int *galois, int M) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= ns / 2) return;
-  const int j = b % stride, i = (b / stride) * 2 * stride;
-  const int st8 = stride << 3, gap = M / st8;
-  const int ti = (galois[j] % st8) * gap;
-  const double2 x = d[i + j], y = cmul(d[i + j + stride], tw[ti]);
-  d[i + j] = dadd2(x, y);
-  d[i + j + stride] = dsub2(x, y);
-}
-
-// BitReverseVector (include/common/CommonUtils.h), out of place
-__global__ void k_bit_reverse(const double2 *src, double2 *dst, int ns, int lb) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= ns) return;
-  dst[__brev(static_cast<unsigned>(i)) >> (32 - lb)] = src[i];
+// The whole special transform of ns = 2^lns slots, bit reversal included:
+// src (overwritten when ns > 1024) -> dst, distinct.
+template <bool INV>
+void special_fft(double2 *src, double2 *dst, int lns, const double2 *tw, const int *galois, int M, cudaStream_t s) {
+  const int in_bits = lns < kFftBits ? lns : kFftBits, out_bits = lns - in_bits;
+  // strides 1 .. 2^(in_bits-1) on 2^in_bits neighbours; the larger ones on
+  // columns of 2^out_bits, 2^(kFftBits-out_bits) of them side by side
+  const int out_cols = kFftBits - out_bits, ctas = 1 << (lns - in_bits);
+  if (INV) {
+    if (out_bits)
+      launch_dependent(k_special_stages<true, false>, ctas, 512, 0, s, static_cast<const double2 *>(src), src, lns, in_bits,
+                       out_bits, out_cols, tw, galois, M);
+    launch_dependent(k_special_stages<true, true>, ctas, 512, 0, s, static_cast<const double2 *>(src), dst, lns, 0, in_bits,
+                     0, tw, galois, M);
+  } else {
+    launch_dependent(k_special_stages<false, true>, ctas, 512, 0, s, static_cast<const double2 *>(src), dst, lns, 0,
+                     in_bits, 0, tw, galois, M);
+    if (out_bits)
+      launch_dependent(k_special_stages<false, false>, ctas, 512, 0, s, static_cast<const double2 *>(dst), dst, lns,
+                       in_bits, out_bits, out_cols, tw, galois, M);
+  }
 }
 
 // round-toward-zero integer of v reduced to [0, p) (BigInt(double) then
@@ -208,9 +250,7 @@ Status Context::encode(int level, double scale, const std::complex<double> *msg,
   for (int i = 0; i < msg_len; i++) h[i] = make_double2(msg[i].real(), msg[i].imag());
   cudaMemcpyAsync(d, h.data(), ns * sizeof(double2), cudaMemcpyHostToDevice, stream);
   const int th = 256;
-  for (int stride = ns / 2; stride >= 1; stride /= 2)
-    k_special_ifft_stage<<<(ns / 2 + th - 1) / th, th, 0, stream>>>(d, ns, stride, d_enc_tw, d_galois, M);
-  k_bit_reverse<<<(ns + th - 1) / th, th, 0, stream>>>(d, e, ns, log2_exact(ns));
+  special_fft<true>(d, e, log2_exact(ns), d_enc_tw, d_galois, M, stream);
   if (gap > 1) cudaMemsetAsync(pt_dev, 0, static_cast<size_t>(tot) * n * 4, stream);
   EncodeRows er{};
   std::vector<int> g(tot);
@@ -273,10 +313,7 @@ Status Context::decode(int level, double scale, const uint32_t *pt_dev, int num_
   for_row_batches(rows, [&](RowBatch &rb) { launch_ntt_inv(rb, P->log_n, stream); });
   const int th = 256;
   k_crt_decode<<<(num_slots + th - 1) / th, th, 0, stream>>>(y, n, gap, num_slots, scale, cr, d);
-  k_bit_reverse<<<(num_slots + th - 1) / th, th, 0, stream>>>(d, e, num_slots, log2_exact(num_slots));
-  for (int stride = 1; stride < num_slots; stride *= 2)
-    k_special_fft_stage<<<(num_slots / 2 + th - 1) / th, th, 0, stream>>>(e, num_slots, stride, d_enc_tw, d_galois,
-                                                                           M);
+  special_fft<false>(d, e, log2_exact(num_slots), d_enc_tw, d_galois, M, stream);
   static_assert(sizeof(std::complex<double>) == sizeof(double2), "complex layout");
   cudaMemcpyAsync(out, e, num_slots * sizeof(double2), cudaMemcpyDeviceToHost, stream);
   return cudaStreamSynchronize(stream) == cudaSuccess ? kOk : check_cuda("decode");
