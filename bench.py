@@ -18,10 +18,8 @@ Reported (one JSON line on rank 0):
   cpu_baseline  the CPU oracle's HMult on the host cores (bounded sample)
   bootstrap  full-slot bootstrapping throughput at N = 2^16 (bootstraps/s;
              decoded precision with real keys: tests/boot_precision_n16.py)
-  ks_engines  the same step with the ModUp / ModDown column passes on each
-             engine (--ks-engine picks the measured one; default auto: the
-             library times both engines on the first launch of each shape
-             and keeps the faster)
+  ks_engines  the same step under each chd_set_ks_engine value (--ks-engine
+             picks the measured one; one column pass serves them all)
   bconv_engines  base conversion on CUDA cores vs tcgen05 tensor cores
   ntt        forward + inverse NTT round trip, 24 primes, HBM fraction
 `--impl reference` times the CPU implementation of the path (the oracle;
@@ -311,14 +309,13 @@ def main():
         "bootstrap": boot, "hoisted_and_mixed": hoist_mixed, "w64": w64, "stream_split": split_cmp,
         "gpu_launches": launches,
     }
-    # the autotuner's choice per column-pass launch shape (largest source
-    # count K, jobs, largest target count M) -> engine / target split
+    # column and row passes whose variant was chosen by timing: none, each
+    # has one variant (the keys stay for readers of earlier lines)
     line["config"]["autotuned_column_passes"] = [
         f"K{t['K']} jobs{t['jobs']} M{t['M']}: "
         f"{({0: 'cuda_core', 1: 'tensor_core', 3: 'tensor_core_wide', 4: 'tensor_core_wide_128regs'}).get(t['engine'], t['engine'])}"
         f"/split{t['split']}"
         for t in chd.ks_tuned_shapes()]
-    # the row pass's choice per shape (ciphertexts, rows, mode) -> variant
     line["config"]["autotuned_row_passes"] = [
         f"cts{t['cts']} rows{t['rows']} mode{t['mode']}: "
         f"{({0: 'in_place_loads', 1: 'prefetch', 2: 'in_place_loads_4ctas'}).get(t['variant'], t['variant'])}"
@@ -535,10 +532,9 @@ def ks_engine_id(chd, args):
 
 
 def ks_engines(ctx, chd, step, stream, steps, B):
-    """The HMult step with the ModUp / ModDown column passes on each engine
-    (CUDA-core int64 BConv vs tcgen05 INT8 byte-limb MMAs); residues are
-    identical (tests), only the time differs.  The one-stream pipeline, so
-    that the stage events time each column pass alone."""
+    """The HMult step under each chd_set_ks_engine value: one column pass
+    serves them all, so the times agree within noise.  The one-stream
+    pipeline, so that the stage events time each column pass alone."""
     import torch
     old = ctx.ks_engine
     ctx.stream_split = False
