@@ -40,11 +40,13 @@ enum RowFlags : uint32_t {
 // parameters under the 32 KiB limit
 constexpr int kMaxRows = 256;
 
-struct RowBatch {
+template <int N>
+struct RowBatchOf {
   int count;
-  uint16_t first[kMaxRows + 1];  // set by the row-phase launches: first limb of each CTA's group
-  RowDesc rows[kMaxRows];
+  uint16_t first[N + 1];  // set by the row-phase launches: first limb of each CTA's group
+  RowDesc rows[N];
 };
+using RowBatch = RowBatchOf<kMaxRows>;
 static_assert(sizeof(RowBatch) + 16 <= 32764, "row batch beyond the kernel parameter limit");
 
 // Forward negacyclic NTT (bit-reversed output) of `count` limbs.
@@ -170,13 +172,15 @@ struct MSColJob {
 // parameters under the 32 KiB limit (a batched ModDown of 30 ciphertexts'
 // 60 polynomials is one launch per stream half)
 constexpr int kMaxMSColJobs = 64;
-struct MSColBatch {
+template <int N>
+struct MSColBatchOf {
   int count;
   const uint2 *tw, *itw;  // twiddle tables [nprimes][N]
   const uint32_t *primes;
   const int32_t *qinvs;
-  MSColJob jobs[kMaxMSColJobs];
+  MSColJob jobs[N];
 };
+using MSColBatch = MSColBatchOf<kMaxMSColJobs>;
 static_assert(sizeof(MSColBatch) + 16 <= 32764, "column-pass batch beyond the kernel parameter limit");
 void launch_modswitch_cols(const MSColBatch &b, int log_n, cudaStream_t s);
 void launch_ntt_inv_rows(RowBatch &rb, int log_n, cudaStream_t s);

@@ -38,6 +38,8 @@
 // the pass is bound by the integer multiplies of the butterflies (8 of the
 // 9.2 cycles a warp needs per butterfly), and what it needs is warps that
 // never wait for one another.
+#include <type_traits>
+
 #include "arith.cuh"
 #include "kernels.h"
 #include "launch.cuh"
@@ -79,8 +81,8 @@ __device__ __forceinline__ uint32_t join(int d0, int d1, int d2, int d3, uint32_
 // Measured, 8 multiplications at level 22 on one stream: ModUp (24 jobs of
 // 8 sources and 24 targets) 85 us, ModDown + Rescale (16 jobs of 9 and 23)
 // 68 us; the 128 x 512 tcgen05 pass before it took 172 and 141 us.
-template <int KR, int MINB>
-__global__ void __launch_bounds__(32 * kColWarps, MINB) k_modswitch_cols(const __grid_constant__ MSColBatch b) {
+template <int KR, int MINB, class B>
+__global__ void __launch_bounds__(32 * kColWarps, MINB) k_modswitch_cols(const __grid_constant__ B b) {
   const MSColJob &jb = b.jobs[blockIdx.y];
   const int lane = threadIdx.x & 31, tq = lane & 3;
   const int col = (blockIdx.x * kColWarps + (threadIdx.x >> 5)) * 8 + (lane >> 2);
@@ -205,18 +207,30 @@ void launch_modswitch_cols(const MSColBatch &b, int log_n, cudaStream_t s) {
   // 25.6 us in two; a multiplication at level 22: 98.7, 103.5 and 107.7 us in
   // one, two and three parts)
   const dim3 grid(kRowLen / kCtaCols, b.count);
-  auto go = [&](auto kern) {
-    // 35 KiB at most (16 sources, 64 targets)
-    launch_dependent(kern, grid, 32 * kColWarps, smem, s, b);
+  // 35 KiB of shared memory at most (16 sources, 64 targets)
+  auto go = [&](const auto &x) {
+    using B = std::decay_t<decltype(x)>;
+    if (max_k <= 4)
+      launch_dependent(k_modswitch_cols<1, 7, B>, grid, 32 * kColWarps, smem, s, x);
+    else if (max_k <= 8)
+      launch_dependent(k_modswitch_cols<2, 6, B>, grid, 32 * kColWarps, smem, s, x);
+    else if (max_k <= 12)
+      launch_dependent(k_modswitch_cols<3, 5, B>, grid, 32 * kColWarps, smem, s, x);
+    else
+      launch_dependent(k_modswitch_cols<4, 4, B>, grid, 32 * kColWarps, smem, s, x);
   };
-  if (max_k <= 4)
-    go(k_modswitch_cols<1, 7>);
-  else if (max_k <= 8)
-    go(k_modswitch_cols<2, 6>);
-  else if (max_k <= 12)
-    go(k_modswitch_cols<3, 5>);
-  else
-    go(k_modswitch_cols<4, 4>);
+  if (b.count > kFewJobs) {
+    go(b);
+    return;
+  }
+  MSColBatchOf<kFewJobs> few;
+  few.count = b.count;
+  few.tw = b.tw;
+  few.itw = b.itw;
+  few.primes = b.primes;
+  few.qinvs = b.qinvs;
+  for (int i = 0; i < b.count; i++) few.jobs[i] = b.jobs[i];
+  go(few);
 }
 
 }  // namespace chd

@@ -19,6 +19,8 @@
 // shared memory).  The inverse runs rows first, then columns, and fuses the
 // per-limb output constant and the optional centring into the column phase.  For N <= 2^15 the whole limb
 // fits in shared memory and one kernel runs every stage.
+#include <type_traits>
+
 #include "arith.cuh"
 #include "kernels.h"
 #include "launch.cuh"
@@ -32,7 +34,8 @@ constexpr int kColThreads = 128;  // columns per CTA of the column phases
 // ---------------------------------------------------------------- N = 2^16
 // Column phase of the forward transform: stages m = 1 .. 8, one column of 16
 // elements per thread.
-__global__ void __launch_bounds__(kColThreads) k_fwd_cols16(const __grid_constant__ RowBatch rb) {
+template <class RB>
+__global__ void __launch_bounds__(kColThreads) k_fwd_cols16(const __grid_constant__ RB rb) {
   const RowDesc &rd = rb.rows[blockIdx.y];
   const uint32_t q = rd.q;
   const int c = blockIdx.x * kColThreads + threadIdx.x;
@@ -54,8 +57,8 @@ __global__ void __launch_bounds__(kColThreads) k_fwd_cols16(const __grid_constan
 // Row phase of the forward transform (input lazy from the column phase),
 // canonical output, with the optional ModDown epilogue (src2 * c1 - x) * c2.
 // A CTA takes one row of one or (P = 2) two limbs of a prime.
-template <int P, int MINB>
-__global__ void __launch_bounds__(kRowThreads, MINB) k_fwd_rows16(const __grid_constant__ RowBatch rb) {
+template <int P, int MINB, class RB>
+__global__ void __launch_bounds__(kRowThreads, MINB) k_fwd_rows16(const __grid_constant__ RB rb) {
   __shared__ __align__(16) uint32_t sm[P][kRowBuf];
   const int first = P == 1 ? blockIdx.y : rb.first[blockIdx.y];
   const bool two = P > 1 && rb.first[blockIdx.y + 1] - first > 1;
@@ -109,8 +112,8 @@ __global__ void __launch_bounds__(kRowThreads, MINB) k_fwd_rows16(const __grid_c
 }
 
 // Inverse, row phase: Gentleman-Sande stages m = 32768 .. 16 (lazy output).
-template <int P, int MINB>
-__global__ void __launch_bounds__(kRowThreads, MINB) k_inv_rows16(const __grid_constant__ RowBatch rb) {
+template <int P, int MINB, class RB>
+__global__ void __launch_bounds__(kRowThreads, MINB) k_inv_rows16(const __grid_constant__ RB rb) {
   __shared__ __align__(16) uint32_t sm[P][kRowBuf];
   const int first = P == 1 ? blockIdx.y : rb.first[blockIdx.y];
   const bool two = P > 1 && rb.first[blockIdx.y + 1] - first > 1;
@@ -150,7 +153,8 @@ __global__ void __launch_bounds__(kRowThreads, MINB) k_inv_rows16(const __grid_c
 }
 
 // Inverse, column phase: stages m = 8 .. 1, then x * c0, canonical or centred.
-__global__ void __launch_bounds__(kColThreads) k_inv_cols16(const __grid_constant__ RowBatch rb) {
+template <class RB>
+__global__ void __launch_bounds__(kColThreads) k_inv_cols16(const __grid_constant__ RB rb) {
   const RowDesc &rd = rb.rows[blockIdx.y];
   const uint32_t q = rd.q;
   const int c = blockIdx.x * kColThreads + threadIdx.x;
@@ -227,9 +231,27 @@ __global__ void __launch_bounds__(1024) k_small(const __grid_constant__ RowBatch
 
 }  // namespace
 
+namespace {
+// go(batch), in a smaller batch when the rows are few (`first` stays unset:
+// only launches of pairs, which are large, read it)
+template <class F>
+void with_rows(const RowBatch &rb, F &&go) {
+  if (rb.count > kFewRows) {
+    go(rb);
+    return;
+  }
+  RowBatchOf<kFewRows> few;
+  few.count = rb.count;
+  for (int i = 0; i < rb.count; i++) few.rows[i] = rb.rows[i];
+  go(few);
+}
+}  // namespace
+
 void launch_ntt_fwd_cols(const RowBatch &rb, int log_n, cudaStream_t s) {
   if (rb.count <= 0) return;
-  launch_dependent(k_fwd_cols16, dim3(kRowLen / kColThreads, rb.count), kColThreads, 0, s, rb);
+  with_rows(rb, [&](const auto &b) {
+    launch_dependent(k_fwd_cols16<std::decay_t<decltype(b)>>, dim3(kRowLen / kColThreads, b.count), kColThreads, 0, s, b);
+  });
 }
 
 namespace {
@@ -256,9 +278,11 @@ void launch_ntt_fwd_rows(RowBatch &rb, int log_n, cudaStream_t s) {
   if (rb.count <= 0) return;
   const int groups = pair_rows(rb);
   if (groups == rb.count || groups * kLimbRows < kPairWaves)
-    launch_dependent(k_fwd_rows16<1, 4>, dim3(kLimbRows, rb.count), kRowThreads, 0, s, rb);
+    with_rows(rb, [&](const auto &b) {
+      launch_dependent(k_fwd_rows16<1, 4, std::decay_t<decltype(b)>>, dim3(kLimbRows, b.count), kRowThreads, 0, s, b);
+    });
   else
-    launch_dependent(k_fwd_rows16<2, 3>, dim3(kLimbRows, groups), kRowThreads, 0, s, rb);
+    launch_dependent(k_fwd_rows16<2, 3, RowBatch>, dim3(kLimbRows, groups), kRowThreads, 0, s, rb);
 }
 
 void launch_ntt_fwd(RowBatch &rb, int log_n, cudaStream_t s) {
@@ -277,16 +301,21 @@ void launch_ntt_inv_rows(RowBatch &rb, int log_n, cudaStream_t s) {
   if (rb.count <= 0) return;
   const int groups = pair_rows(rb);
   if (groups == rb.count || groups * kLimbRows < kPairWaves)
-    launch_dependent(k_inv_rows16<1, 4>, dim3(kLimbRows, rb.count), kRowThreads, 0, s, rb);
+    with_rows(rb, [&](const auto &b) {
+      launch_dependent(k_inv_rows16<1, 4, std::decay_t<decltype(b)>>, dim3(kLimbRows, b.count), kRowThreads, 0, s, b);
+    });
   else
-    launch_dependent(k_inv_rows16<2, 3>, dim3(kLimbRows, groups), kRowThreads, 0, s, rb);
+    launch_dependent(k_inv_rows16<2, 3, RowBatch>, dim3(kLimbRows, groups), kRowThreads, 0, s, rb);
 }
 
 void launch_ntt_inv(RowBatch &rb, int log_n, cudaStream_t s) {
   if (rb.count <= 0) return;
   if (log_n == 16) {
     launch_ntt_inv_rows(rb, log_n, s);
-    launch_dependent(k_inv_cols16, dim3(kRowLen / kColThreads, rb.count), kColThreads, 0, s, rb);
+    with_rows(rb, [&](const auto &b) {
+      launch_dependent(k_inv_cols16<std::decay_t<decltype(b)>>, dim3(kRowLen / kColThreads, b.count), kColThreads, 0, s,
+                       b);
+    });
   } else {
     size_t smem = sizeof(uint32_t) << log_n;
     cudaFuncSetAttribute(k_small<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024);
