@@ -546,7 +546,10 @@ void Arena::release(size_t m) { top_ = m; }
 // -------------------------------------------------------------- Context
 std::unique_ptr<Context> Context::create(const ParamSpec &spec, int device, std::string *err) {
   auto c = std::unique_ptr<Context>(new Context());
-  if (c->init(spec, device, err) != kOk) return nullptr;
+  if (c->init(spec, device, err) != kOk) {
+    cudaGetLastError();  // reported here: not to be taken for the next call's
+    return nullptr;
+  }
   return c;
 }
 
@@ -673,12 +676,18 @@ void epi_consts(const std::vector<uint32_t> &src, const std::vector<uint32_t> &d
     (*pad)[i] = prime::to_mont(v, p);
   }
 }
-int32_t *upload_i32(const std::vector<int32_t> &v) {
-  int32_t *p = nullptr;
-  if (v.empty()) return nullptr;
-  if (cudaMalloc(&p, v.size() * 4) != cudaSuccess) return nullptr;
-  cudaMemcpy(p, v.data(), v.size() * 4, cudaMemcpyHostToDevice);
-  return p;
+// Device copy of a host table: *out stays null for an empty one.  False when
+// there is no memory for it or the copy fails, which the caller must not take
+// for the null of an empty table.
+template <typename T>
+bool upload(const std::vector<T> &v, T **out) {
+  *out = nullptr;
+  if (v.empty()) return true;
+  if (cudaMalloc(out, v.size() * sizeof(T)) != cudaSuccess) {
+    *out = nullptr;
+    return false;
+  }
+  return cudaMemcpy(*out, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice) == cudaSuccess;
 }
 
 // B fragments of the column pass's base-conversion MMAs (modswitch.cu) for a
@@ -688,8 +697,10 @@ int32_t *upload_i32(const std::vector<int32_t> &v) {
 // target nn / 2 of the group and source tq / tq + 4 of the step, .z / .w the
 // same of byte i + 2; zero past the last target or source.  After the steps
 // one uint4 per lane holds the four bytes of -2^30 sum_k T mod p of target tq.
-uint4 *upload_frags(const std::vector<int32_t> &T, int K, int M, const uint32_t *p) {
-  if (T.empty() || K < 1 || K > 16) return nullptr;
+// No table (null) for shapes that the column pass refuses; false as upload().
+bool upload_frags(const std::vector<int32_t> &T, int K, int M, const uint32_t *p, uint4 **out) {
+  *out = nullptr;
+  if (T.empty() || K < 1 || K > 16) return true;
   const int groups = (M + 3) / 4, steps = (K + 7) / 8;
   std::vector<uint4> f(static_cast<size_t>(groups) * (steps + 1) * 32, make_uint4(0, 0, 0, 0));
   auto plain = [&](int m, int k) {
@@ -720,10 +731,7 @@ uint4 *upload_frags(const std::vector<int32_t> &T, int K, int M, const uint32_t 
       }
     }
   }
-  uint4 *d = nullptr;
-  if (cudaMalloc(&d, f.size() * sizeof(uint4)) != cudaSuccess) return nullptr;
-  cudaMemcpy(d, f.data(), f.size() * sizeof(uint4), cudaMemcpyHostToDevice);
-  return d;
+  return upload(f, out);
 }
 }  // namespace
 
@@ -890,10 +898,14 @@ Status Context::init(const ParamSpec &spec, int dev, std::string *err) {
   for (int level = -1; level <= P->max_level; level++) {
     LevelMS &m = ms[level + 1];
     build_level_ms(*P, level, &m);
-    for (auto &t : m.mod_up2) m.d_mod_up2.push_back(t.empty() ? nullptr : upload_i32(t));
-    m.d_mod_down2 = upload_i32(m.mod_down2);
-    m.d_rs2 = upload_i32(m.rs2);
-    m.d_mdr2 = upload_i32(m.mdr2);
+    bool ok = true;
+    m.d_mod_up2.assign(m.mod_up2.size(), nullptr);
+    for (size_t i = 0; i < m.mod_up2.size(); i++) ok = ok && upload(m.mod_up2[i], &m.d_mod_up2[i]);
+    ok = ok && upload(m.mod_down2, &m.d_mod_down2) && upload(m.rs2, &m.d_rs2) && upload(m.mdr2, &m.d_mdr2);
+    if (!ok) {
+      *err = "device allocation failed";
+      return kErrAlloc;
+    }
     if (P->log_n != 16) continue;
     // targets: the extended basis without the digit's own primes (ModUp), the
     // level's q primes (ModDown), the next level's (Rescale, merged)
@@ -902,21 +914,27 @@ Status Context::init(const ParamSpec &spec, int dev, std::string *err) {
     P->gidx(np, g.data());
     std::vector<uint32_t> lp;
     for (int x : g) lp.push_back(P->primes[x]);
+    m.d_mod_up_frag.assign(m.beta, nullptr);
     for (int i = 0; i < m.beta; i++) {
       std::vector<uint32_t> dst(lp.begin(), lp.begin() + m.dig_s[i]);
       dst.insert(dst.end(), lp.begin() + m.dig_e[i], lp.end());
-      m.d_mod_up_frag.push_back(
-          upload_frags(m.mod_up2[i], m.dig_e[i] - m.dig_s[i], static_cast<int>(dst.size()), dst.data()));
+      ok = ok && upload_frags(m.mod_up2[i], m.dig_e[i] - m.dig_s[i], static_cast<int>(dst.size()), dst.data(),
+                              &m.d_mod_up_frag[i]);
     }
-    m.d_mod_down_frag = upload_frags(m.mod_down2, np.aux, np.q(), lp.data());
-    if (!m.has_rescale) continue;
-    const NP nn = P->level_np(level - 1, 0);
-    std::vector<int> gn(nn.total());
-    P->gidx(nn, gn.data());
-    std::vector<uint32_t> next;
-    for (int x : gn) next.push_back(P->primes[x]);
-    m.d_rs_frag = upload_frags(m.rs2, m.rs_src_len, nn.q(), next.data());
-    m.d_mdr_frag = upload_frags(m.mdr2, m.mdr_src_len, nn.q(), next.data());
+    ok = ok && upload_frags(m.mod_down2, np.aux, np.q(), lp.data(), &m.d_mod_down_frag);
+    if (m.has_rescale) {
+      const NP nn = P->level_np(level - 1, 0);
+      std::vector<int> gn(nn.total());
+      P->gidx(nn, gn.data());
+      std::vector<uint32_t> next;
+      for (int x : gn) next.push_back(P->primes[x]);
+      ok = ok && upload_frags(m.rs2, m.rs_src_len, nn.q(), next.data(), &m.d_rs_frag) &&
+           upload_frags(m.mdr2, m.mdr_src_len, nn.q(), next.data(), &m.d_mdr_frag);
+    }
+    if (!ok) {
+      *err = "device allocation failed";
+      return kErrAlloc;
+    }
   }
   if (cudaDeviceSynchronize() != cudaSuccess) {
     *err = std::string("context setup: ") + cudaGetErrorString(cudaGetLastError());
@@ -1238,7 +1256,7 @@ Status Context::modup_fused(int level, int count, const uint32_t *const *src, ui
       j.frag = m.d_mod_up_frag[i];
       j.K = e - s;
       j.M = tot - (e - s);
-      CHD_CHECK(j.K <= 16 && j.M <= 64, kErrUnsupported, "modup: digit too large");
+      CHD_CHECK(j.frag && j.K <= 16 && j.M <= 64, kErrUnsupported, "modup: digit too large");
       for (int k = 0; k < j.K; k++) {
         j.src_row[k] = static_cast<uint8_t>(s + k);
         j.src_gidx[k] = static_cast<uint8_t>(g[s + k]);
@@ -1285,6 +1303,7 @@ Status Context::moddown_plan(int level, MDType type, MDPlan *pl) const {
   CHD_CHECK(pl->src_len >= 1 && pl->src_len <= 16, kErrUnsupported, "moddown: more than 16 dropped primes");
   pl->c1 = type == MDType::kModDown ? m.mod_down1.data() : type == MDType::kRescale ? m.rs1.data() : m.mdr1.data();
   pl->frag = type == MDType::kModDown ? m.d_mod_down_frag : type == MDType::kRescale ? m.d_rs_frag : m.d_mdr_frag;
+  CHD_CHECK(pl->frag, kErrUnsupported, "moddown: no conversion table for this shape");
   pl->inv = type == MDType::kModDown ? m.inv_p_prod.data() : type == MDType::kRescale ? m.rs_inv.data() : m.mdr_inv.data();
   pl->pad = type == MDType::kModDown ? nullptr : type == MDType::kRescale ? m.rs_pad.data() : m.mdr_pad.data();
   pl->gs.assign(pl->ns.total(), 0);
@@ -1450,7 +1469,7 @@ Status Context::key_switch_fused_pipeline(const int *levels, int count, const KS
         j.frag = m.d_mod_up_frag[i];
         j.K = e - s;
         j.M = sh.tot - (e - s);
-        CHD_CHECK(j.K <= 16 && j.M <= 64, kErrUnsupported, "modup: digit too large");
+        CHD_CHECK(j.frag && j.K <= 16 && j.M <= 64, kErrUnsupported, "modup: digit too large");
         for (int k = 0; k < j.K; k++) {
           j.src_row[k] = static_cast<uint8_t>(s + k);
           j.src_gidx[k] = static_cast<uint8_t>(sh.g[s + k]);
@@ -1679,6 +1698,7 @@ Status Context::moddown_pipeline(int level, MDType type, const uint32_t *const *
   const int32_t *table = type == MDType::kModDown ? m.d_mod_down2 : type == MDType::kRescale ? m.d_rs2 : m.d_mdr2;
   const uint4 *frag = type == MDType::kModDown  ? m.d_mod_down_frag
                       : type == MDType::kRescale ? m.d_rs_frag : m.d_mdr_frag;
+  CHD_CHECK(frag || P->log_n != 16, kErrUnsupported, "moddown: no conversion table for this shape");
   const uint32_t *inv = type == MDType::kModDown ? m.inv_p_prod.data()
                         : type == MDType::kRescale ? m.rs_inv.data() : m.mdr_inv.data();
   const uint32_t *pad = type == MDType::kModDown ? nullptr

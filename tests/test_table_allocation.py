@@ -1,0 +1,119 @@
+"""Device memory that runs out while a context builds its constant tables.
+
+Runs without a GPU: the library's process gets a stand-in for the CUDA runtime
+(preloaded, host memory for device memory) that refuses the n-th allocation
+and counts kernel launches.  A context must be refused whichever allocation
+fails, never come up with a table missing, and give back what it had taken;
+whatever is refused must also leave the next call, with memory again, intact.
+"""
+import os
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+PKG = os.path.join(os.path.dirname(HERE), "cheddar-fhe_b200")
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+
+RUNTIME = r'''
+#include <cuda_runtime_api.h>
+#include <stdlib.h>
+#include <string.h>
+static long mallocs, live, fail_at = -1, launches;
+static cudaError_t last;
+long fake_mallocs(void) { return mallocs; }
+long fake_live(void) { return live; }
+long fake_launches(void) { return launches; }
+int fake_last(void) { return last; }
+void fake_reset(long n) { mallocs = launches = 0; fail_at = n; }
+static cudaError_t ok(void) { return cudaSuccess; }
+cudaError_t cudaMalloc(void **p, size_t n) {
+  if (mallocs++ == fail_at) return last = cudaErrorMemoryAllocation;
+  *p = calloc(1, n);
+  live++;
+  return ok();
+}
+cudaError_t cudaFree(void *p) { if (p) live--; free(p); return ok(); }
+cudaError_t cudaMemcpy(void *d, const void *s, size_t n, enum cudaMemcpyKind k) { memcpy(d, s, n); return ok(); }
+cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, enum cudaMemcpyKind k, cudaStream_t t) {
+  memmove(d, s, n);
+  return ok();
+}
+cudaError_t cudaMemset(void *d, int v, size_t n) { memset(d, v, n); return ok(); }
+cudaError_t cudaMemsetAsync(void *d, int v, size_t n, cudaStream_t s) { memset(d, v, n); return ok(); }
+cudaError_t cudaSetDevice(int d) { return ok(); }
+cudaError_t cudaGetDevice(int *d) { *d = 0; return ok(); }
+cudaError_t cudaDeviceGetAttribute(int *v, enum cudaDeviceAttr a, int d) { *v = 148; return ok(); }
+cudaError_t cudaDeviceSynchronize(void) { return ok(); }
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned f) { *s = (cudaStream_t)malloc(1); return ok(); }
+cudaError_t cudaStreamDestroy(cudaStream_t s) { free(s); return ok(); }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) { return ok(); }
+cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned f) { return ok(); }
+cudaError_t cudaStreamIsCapturing(cudaStream_t s, enum cudaStreamCaptureStatus *c) { *c = 0; return ok(); }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned f) { *e = (cudaEvent_t)malloc(1); return ok(); }
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) { return ok(); }
+cudaError_t cudaEventDestroy(cudaEvent_t e) { free(e); return ok(); }
+cudaError_t cudaGetLastError(void) { cudaError_t e = last; last = cudaSuccess; return e; }
+cudaError_t cudaFuncSetAttribute(const void *f, enum cudaFuncAttribute a, int v) { return ok(); }
+cudaError_t cudaLaunchKernel(const void *f, dim3 g, dim3 b, void **a, size_t m, cudaStream_t s) {
+  launches++;
+  return ok();
+}
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void **a) { launches++; return ok(); }
+'''
+
+PRELUDE = f"""
+import ctypes as C, json, os, sys
+sys.path.insert(0, {PKG!r})
+import cheddar_b200 as chd
+rt = C.CDLL(None)
+for f in ("fake_mallocs", "fake_live", "fake_launches"):
+    getattr(rt, f).restype = C.c_long
+rt.fake_reset.argtypes = [C.c_long]
+
+def refused(make):
+    try:
+        return None, make()
+    except chd.CheddarError as e:
+        return str(e), None
+"""
+
+
+@pytest.fixture(scope="module")
+def runtime(tmp_path_factory):
+    d = tmp_path_factory.mktemp("runtime")
+    src, so = d / "runtime.c", d / "runtime.so"
+    src.write_text(RUNTIME)
+    subprocess.run(["gcc", "-shared", "-fPIC", "-O1", "-w", f"-I{CUDA}/include", "-o", str(so), str(src)], check=True)
+
+    def run(body):
+        r = subprocess.run([sys.executable, "-c", PRELUDE + textwrap.dedent(body)], capture_output=True, text=True,
+                           timeout=600, env=dict(os.environ, LD_PRELOAD=str(so)))
+        assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-3000:]
+
+    return run
+
+
+def test_context_is_refused_whichever_allocation_fails(runtime):
+    # three primes of digits 1 wide: every table kind of N = 2^16 and of a
+    # smaller degree, over three levels and a rescale
+    runtime("""
+        p = json.load(open(os.path.join(chd.PARAM_DIR, "keyswitch_l8_a3.json")))
+        p.update(main_primes=p["main_primes"][:3], auxiliary_primes=p["auxiliary_primes"][:1],
+                 level_config=[[i, 0] for i in range(1, 4)], default_encryption_level=0)
+        for log_n in (16, 12):
+            text = json.dumps(dict(p, log_degree=log_n))
+            rt.fake_reset(-1)
+            ctx = chd.Context(text)
+            total = rt.fake_mallocs()
+            assert total >= 15 and rt.fake_live() == total
+            ctx.close()
+            assert rt.fake_live() == 0
+            for n in range(total):
+                rt.fake_reset(n)
+                err, ctx = refused(lambda: chd.Context(text))
+                assert err and "allocation" in err, (log_n, n, err)
+                assert rt.fake_live() == 0 and rt.fake_last() == 0, (log_n, n)
+    """)
