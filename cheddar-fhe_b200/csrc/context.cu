@@ -899,14 +899,16 @@ Status Context::init(const ParamSpec &spec, int dev, std::string *err) {
     LevelMS &m = ms[level + 1];
     build_level_ms(*P, level, &m);
     bool ok = true;
-    m.d_mod_up2.assign(m.mod_up2.size(), nullptr);
-    for (size_t i = 0; i < m.mod_up2.size(); i++) ok = ok && upload(m.mod_up2[i], &m.d_mod_up2[i]);
-    ok = ok && upload(m.mod_down2, &m.d_mod_down2) && upload(m.rs2, &m.d_rs2) && upload(m.mdr2, &m.d_mdr2);
-    if (!ok) {
-      *err = "device allocation failed";
-      return kErrAlloc;
+    if (P->log_n != 16) {  // the unfused base conversion reads the tables themselves
+      m.d_mod_up2.assign(m.mod_up2.size(), nullptr);
+      for (size_t i = 0; i < m.mod_up2.size(); i++) ok = ok && upload(m.mod_up2[i], &m.d_mod_up2[i]);
+      ok = ok && upload(m.mod_down2, &m.d_mod_down2) && upload(m.rs2, &m.d_rs2) && upload(m.mdr2, &m.d_mdr2);
+      if (!ok) {
+        *err = "device allocation failed";
+        return kErrAlloc;
+      }
+      continue;
     }
-    if (P->log_n != 16) continue;
     // targets: the extended basis without the digit's own primes (ModUp), the
     // level's q primes (ModDown), the next level's (Rescale, merged)
     const NP np = P->level_np(level, m.num_aux);
@@ -1695,7 +1697,6 @@ Status Context::moddown_pipeline(int level, MDType type, const uint32_t *const *
   CHD_CHECK(src_len >= 1 && src_len <= 16, kErrUnsupported, "moddown: more than 16 dropped primes");
   const uint32_t *c1 = type == MDType::kModDown ? m.mod_down1.data()
                        : type == MDType::kRescale ? m.rs1.data() : m.mdr1.data();
-  const int32_t *table = type == MDType::kModDown ? m.d_mod_down2 : type == MDType::kRescale ? m.d_rs2 : m.d_mdr2;
   const uint4 *frag = type == MDType::kModDown  ? m.d_mod_down_frag
                       : type == MDType::kRescale ? m.d_rs_frag : m.d_mdr_frag;
   CHD_CHECK(frag || P->log_n != 16, kErrUnsupported, "moddown: no conversion table for this shape");
@@ -1766,6 +1767,7 @@ Status Context::moddown_pipeline(int level, MDType type, const uint32_t *const *
     launch_modswitch_cols(b, P->log_n, stream);
   } else {
     for_row_batches(rows, [&](RowBatch &rb) { launch_ntt_inv(rb, P->log_n, stream); });
+    const int32_t *table = type == MDType::kModDown ? m.d_mod_down2 : type == MDType::kRescale ? m.d_rs2 : m.d_mdr2;
     BConvBatch b{};
     b.primes = d_primes;
     b.qinvs = d_qinv;

@@ -115,10 +115,10 @@ struct LevelMS {
   int rs_src_len = 0, mdr_src_len = 0, rs_dst_len = 0;
   std::vector<uint32_t> rs1, rs_inv, rs_pad, mdr1, mdr_inv, mdr_pad;
   std::vector<int32_t> rs2, mdr2;
-  // device copies of the BConv tables
+  // N < 2^16: device copies of the BConv tables
   std::vector<int32_t *> d_mod_up2;
   int32_t *d_mod_down2 = nullptr, *d_rs2 = nullptr, *d_mdr2 = nullptr;
-  // N = 2^16: the same tables as MMA fragments of the fused column pass
+  // N = 2^16: the tables as MMA fragments of the fused column pass
   std::vector<uint4 *> d_mod_up_frag;
   uint4 *d_mod_down_frag = nullptr, *d_rs_frag = nullptr, *d_mdr_frag = nullptr;
 };
