@@ -533,7 +533,10 @@ void *Arena::alloc(size_t bytes) {
   }
   size_t sz = std::max(bytes, total_ ? total_ : static_cast<size_t>(64) << 20);
   char *p = nullptr;
-  if (cudaMalloc(&p, sz) != cudaSuccess) return nullptr;
+  if (cudaMalloc(&p, sz) != cudaSuccess) {
+    cudaGetLastError();  // the caller reports it: not to be taken for the next call's
+    return nullptr;
+  }
   chunks_.push_back(Chunk{p, sz, total_});
   top_ = total_ + bytes;
   total_ += sz;

@@ -313,12 +313,16 @@ void epi_consts(const std::vector<u64> &src, const std::vector<u64> &dst, int rs
     (*pad)[i] = to_mont(v, p);
   }
 }
-i64 *upload(const std::vector<i64> &v) {
-  i64 *p = nullptr;
-  if (v.empty()) return nullptr;
-  if (cudaMalloc(&p, v.size() * 8) != cudaSuccess) return nullptr;
-  cudaMemcpy(p, v.data(), v.size() * 8, cudaMemcpyHostToDevice);
-  return p;
+// Device copy of a host table, in order with the work of `s`: *out stays null
+// for an empty one; false when there is no memory for it or the copy fails
+bool upload(const std::vector<i64> &v, cudaStream_t s, i64 **out) {
+  *out = nullptr;
+  if (v.empty()) return true;
+  if (cudaMalloc(out, v.size() * 8) != cudaSuccess) {
+    *out = nullptr;
+    return false;
+  }
+  return cudaMemcpyAsync(*out, v.data(), v.size() * 8, cudaMemcpyHostToDevice, s) == cudaSuccess;
 }
 }  // namespace
 
@@ -441,15 +445,16 @@ Evk64::~Evk64() {
   cudaFree(ax);
 }
 
+LevelMS64::~LevelMS64() {
+  for (auto *t : d_mod_up2) cudaFree(t);
+  cudaFree(d_mod_down2);
+  cudaFree(d_rs2);
+  cudaFree(d_mdr2);
+}
+
 Context64::~Context64() {
   if (P) cudaSetDevice(device);
-  for (auto &m : ms)
-    if (m) {
-      for (auto *t : m->d_mod_up2) cudaFree(t);
-      cudaFree(m->d_mod_down2);
-      cudaFree(m->d_rs2);
-      cudaFree(m->d_mdr2);
-    }
+  ms.clear();
   cudaFree(d_primes);
   cudaFree(d_qinv);
   cudaFree(d_tw);
@@ -544,20 +549,31 @@ Status Context64::init(const ParamSpec64 &spec, int dev, std::string *err) {
     p_prod[i] = to_mont(v, q);
   }
   ms.resize(P->max_level + 2);
+  // a copy from pageable memory may return before it has reached the device,
+  // and the context's stream does not wait for it
+  cudaDeviceSynchronize();
   return check("context64 init");
 }
 
-const LevelMS64 &Context64::lms(int level) {
+const LevelMS64 *Context64::lms(int level) {
   auto &slot = ms.at(level + 1);
   if (!slot) {
-    slot = std::make_unique<LevelMS64>();
-    build_level_ms64(*P, level, slot.get());
-    for (auto &t : slot->mod_up2) slot->d_mod_up2.push_back(t.empty() ? nullptr : upload(t));
-    slot->d_mod_down2 = upload(slot->mod_down2);
-    slot->d_rs2 = upload(slot->rs2);
-    slot->d_mdr2 = upload(slot->mdr2);
+    auto m = std::make_unique<LevelMS64>();
+    build_level_ms64(*P, level, m.get());
+    m->d_mod_up2.assign(m->mod_up2.size(), nullptr);
+    bool ok = true;
+    for (size_t i = 0; i < m->mod_up2.size(); i++) ok = ok && upload(m->mod_up2[i], stream, &m->d_mod_up2[i]);
+    ok = ok && upload(m->mod_down2, stream, &m->d_mod_down2) && upload(m->rs2, stream, &m->d_rs2) &&
+         upload(m->mdr2, stream, &m->d_mdr2);
+    // complete before use: k64_bconv reads its table ahead of the kernels before it
+    if (cudaStreamSynchronize(stream) != cudaSuccess || !ok) {
+      cudaGetLastError();
+      set_error("64-bit level constants: device allocation or copy failed");
+      return nullptr;
+    }
+    slot = std::move(m);
   }
-  return *slot;
+  return slot.get();
 }
 
 namespace {
@@ -619,7 +635,9 @@ Status Context64::modup(int level, const u64 *src, u64 *dst) {
   // ModSwitchHandler::ModUp (ModSwitch.cu:429-509): INTT of the q limbs times
   // the digit constants (centred), per digit a copy of its own limbs, the
   // base conversion to the other primes and their NTT
-  const LevelMS64 &m = lms(level);
+  const LevelMS64 *lm = lms(level);
+  if (!lm) return kErrAlloc;
+  const LevelMS64 &m = *lm;
   const int n = P->n;
   const NP np = P->level_np(level, m.num_aux);
   const int nq = np.q(), tot = np.total();
@@ -686,7 +704,9 @@ Status Context64::modup(int level, const u64 *src, u64 *dst) {
 Status Context64::moddown(int level, MDType type, const u64 *const *src, u64 *const *dst, int npoly) {
   // ModSwitch.cu:566-684 with the NTT epilogue of NTT.cu:456-601 (word =
   // uint64_t)
-  const LevelMS64 &m = lms(level);
+  const LevelMS64 *lm = lms(level);
+  if (!lm) return kErrAlloc;
+  const LevelMS64 &m = *lm;
   const int n = P->n;
   CHD_CHECK(type == MDType::kModDown || m.has_rescale, kErrInvalidLevel, "rescale not available at this level");
   const int nsa = type == MDType::kRescale ? 0 : m.num_aux;
@@ -784,7 +804,9 @@ Status Context64::key_mult(int level, const u64 *d, const u64 *d0, const u64 *d1
   // MultKeyNoModDown (Context.cpp:609-648): ModUp of d, then the inner
   // product with the key's digits over Q u P, plus P (d0, d1) on the q rows
   // (the CAccum of Context.cpp:687-699)
-  const LevelMS64 &m = lms(level);
+  const LevelMS64 *lm = lms(level);
+  if (!lm) return kErrAlloc;
+  const LevelMS64 &m = *lm;
   const int n = P->n;
   const NP np = P->level_np(level, P->alpha);
   const int nq = np.q(), tot = np.total();
@@ -1471,8 +1493,9 @@ int chd64_moddown_raw(chd64_context *ctx, int level, int type, const uint64_t *s
     return fail64(CHD_ERR_INVALID_ARG, "chd64_moddown_raw: invalid type");
   const MDType t = type == CHD_MODDOWN ? MDType::kModDown : type == CHD_RESCALE ? MDType::kRescale
                                                                                    : MDType::kModDownRescale;
-  const LevelMS64 &m = C.lms(level);
-  const NP ns = C.P->level_np(level, t == MDType::kRescale ? 0 : m.num_aux);
+  const LevelMS64 *m = C.lms(level);
+  if (!m) return CHD_ERR_ALLOC;
+  const NP ns = C.P->level_np(level, t == MDType::kRescale ? 0 : m->num_aux);
   const NP nd = C.P->level_np(t == MDType::kModDown ? level : level - 1, 0);
   if (t != MDType::kModDown && level < 1) return fail64(CHD_ERR_INVALID_LEVEL, "chd64_moddown_raw: no rescale at level 0");
   std::vector<const uint64_t *> s(npoly);

@@ -69,6 +69,10 @@ struct LevelMS64 {
   std::vector<i64> rs2, mdr2;
   std::vector<i64 *> d_mod_up2;
   i64 *d_mod_down2 = nullptr, *d_rs2 = nullptr, *d_mdr2 = nullptr;
+  LevelMS64() = default;
+  LevelMS64(const LevelMS64 &) = delete;
+  LevelMS64 &operator=(const LevelMS64 &) = delete;
+  ~LevelMS64();
 };
 void build_level_ms64(const Params64 &P, int level, LevelMS64 *m);
 
@@ -115,7 +119,7 @@ class Context64 {
   bool narrow = false;  // every prime below 2^58 (k64_bconv)
   std::vector<u64> p_prod;  // Montgomery P mod q_i for the q primes of the key basis
   std::vector<std::unique_ptr<LevelMS64>> ms;  // index level + 1
-  const LevelMS64 &lms(int level);
+  const LevelMS64 *lms(int level);  // null, with the error set, when there is no memory for the tables
   const ulonglong2 *tw(int g) const { return d_tw + (static_cast<size_t>(g) << P->log_n); }
   const ulonglong2 *itw(int g) const { return d_itw + (static_cast<size_t>(g) << P->log_n); }
   void shoup(u64 c, int g, u64 *w, u64 *ws) const;       // plain constant c

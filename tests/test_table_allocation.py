@@ -5,6 +5,9 @@ Runs without a GPU: the library's process gets a stand-in for the CUDA runtime
 and counts kernel launches.  A context must be refused whichever allocation
 fails, never come up with a table missing, and give back what it had taken;
 whatever is refused must also leave the next call, with memory again, intact.
+The stand-in also counts launches that come after a copy from pageable host
+memory (which may return early, and which other streams do not wait for) and
+before a synchronisation.
 """
 import os
 import subprocess
@@ -21,13 +24,14 @@ RUNTIME = r'''
 #include <cuda_runtime_api.h>
 #include <stdlib.h>
 #include <string.h>
-static long mallocs, live, fail_at = -1, launches;
+static long mallocs, live, fail_at = -1, launches, copying, early;
 static cudaError_t last;
 long fake_mallocs(void) { return mallocs; }
 long fake_live(void) { return live; }
 long fake_launches(void) { return launches; }
+long fake_early(void) { return early; }
 int fake_last(void) { return last; }
-void fake_reset(long n) { mallocs = launches = 0; fail_at = n; }
+void fake_reset(long n) { mallocs = launches = early = 0; fail_at = n; }
 static cudaError_t ok(void) { return cudaSuccess; }
 cudaError_t cudaMalloc(void **p, size_t n) {
   if (mallocs++ == fail_at) return last = cudaErrorMemoryAllocation;
@@ -36,7 +40,11 @@ cudaError_t cudaMalloc(void **p, size_t n) {
   return ok();
 }
 cudaError_t cudaFree(void *p) { if (p) live--; free(p); return ok(); }
-cudaError_t cudaMemcpy(void *d, const void *s, size_t n, enum cudaMemcpyKind k) { memcpy(d, s, n); return ok(); }
+cudaError_t cudaMemcpy(void *d, const void *s, size_t n, enum cudaMemcpyKind k) {
+  memcpy(d, s, n);
+  copying |= k == cudaMemcpyHostToDevice;
+  return ok();
+}
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, enum cudaMemcpyKind k, cudaStream_t t) {
   memmove(d, s, n);
   return ok();
@@ -46,7 +54,7 @@ cudaError_t cudaMemsetAsync(void *d, int v, size_t n, cudaStream_t s) { memset(d
 cudaError_t cudaSetDevice(int d) { return ok(); }
 cudaError_t cudaGetDevice(int *d) { *d = 0; return ok(); }
 cudaError_t cudaDeviceGetAttribute(int *v, enum cudaDeviceAttr a, int d) { *v = 148; return ok(); }
-cudaError_t cudaDeviceSynchronize(void) { return ok(); }
+cudaError_t cudaDeviceSynchronize(void) { copying = 0; return ok(); }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned f) { *s = (cudaStream_t)malloc(1); return ok(); }
 cudaError_t cudaStreamDestroy(cudaStream_t s) { free(s); return ok(); }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) { return ok(); }
@@ -59,17 +67,23 @@ cudaError_t cudaGetLastError(void) { cudaError_t e = last; last = cudaSuccess; r
 cudaError_t cudaFuncSetAttribute(const void *f, enum cudaFuncAttribute a, int v) { return ok(); }
 cudaError_t cudaLaunchKernel(const void *f, dim3 g, dim3 b, void **a, size_t m, cudaStream_t s) {
   launches++;
+  early += copying;
   return ok();
 }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void **a) { launches++; return ok(); }
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void **a) {
+  launches++;
+  early += copying;
+  return ok();
+}
 '''
 
 PRELUDE = f"""
 import ctypes as C, json, os, sys
+import numpy as np
 sys.path.insert(0, {PKG!r})
 import cheddar_b200 as chd
 rt = C.CDLL(None)
-for f in ("fake_mallocs", "fake_live", "fake_launches"):
+for f in ("fake_mallocs", "fake_live", "fake_launches", "fake_early"):
     getattr(rt, f).restype = C.c_long
 rt.fake_reset.argtypes = [C.c_long]
 
@@ -116,4 +130,35 @@ def test_context_is_refused_whichever_allocation_fails(runtime):
                 err, ctx = refused(lambda: chd.Context(text))
                 assert err and "allocation" in err, (log_n, n, err)
                 assert rt.fake_live() == 0 and rt.fake_last() == 0, (log_n, n)
+    """)
+
+
+def test_level_constants_of_the_64_bit_path(runtime):
+    # built on first use: ModUp and ModDown + Rescale fail with the
+    # allocation, launch nothing, and work once there is memory
+    runtime("""
+        p = json.load(open(os.path.join(chd.PARAM_DIR, "bootparam_40_64bit.json")))
+        p.update(main_primes=p["main_primes"][:3], auxiliary_primes=p["auxiliary_primes"][:2],
+                 level_config=[[i, 0] for i in range(1, 4)], default_encryption_level=0)
+        src, ext = np.zeros((5, 65536), np.uint64), np.zeros((2, 5, 65536), np.uint64)
+        calls = [lambda c: c.modup_raw(2, src.ctypes.data, ext.ctypes.data),
+                 lambda c: c.moddown_raw(2, chd.CHD_MODDOWN_RESCALE, src.ctypes.data, ext.ctypes.data)]
+        for call in calls:
+            total = 1
+            n = -1
+            while n < total:
+                rt.fake_reset(-1)
+                ctx = chd.Context64(json.dumps(p))
+                rt.fake_reset(n)
+                err, _ = refused(lambda: call(ctx))
+                if n < 0:
+                    total = rt.fake_mallocs()
+                    assert total >= 5 and err is None
+                elif n < total:
+                    assert err and "failed" in err and rt.fake_launches() == 0, (n, err)
+                    rt.fake_reset(-1)
+                    call(ctx)
+                assert rt.fake_launches() > 0 and rt.fake_early() == 0
+                del ctx
+                n += 1
     """)
