@@ -218,14 +218,16 @@ int log2_exact(int x) {
 }  // namespace
 
 Status Context::codec_tables() {
-  if (d_enc_tw) return kOk;
+  if (d_enc_tw && d_galois) return kOk;
   const auto &tw = enc_twiddles();
-  CHD_CHECK(cudaMalloc(&d_enc_tw, tw.size() * sizeof(double2)) == cudaSuccess, kErrAlloc,
-            "encoder: twiddle table allocation failed");
-  CHD_CHECK(cudaMalloc(&d_galois, P->galois.size() * sizeof(int)) == cudaSuccess, kErrAlloc,
-            "encoder: galois table allocation failed");
-  cudaMemcpy(d_enc_tw, tw.data(), tw.size() * sizeof(double2), cudaMemcpyHostToDevice);
-  cudaMemcpy(d_galois, P->galois.data(), P->galois.size() * sizeof(int), cudaMemcpyHostToDevice);
+  // either may be there already, from a call that had no memory for the other
+  const bool ok = (d_enc_tw || cudaMalloc(&d_enc_tw, tw.size() * sizeof(double2)) == cudaSuccess) &&
+                  (d_galois || cudaMalloc(&d_galois, P->galois.size() * sizeof(int)) == cudaSuccess);
+  if (!ok) cudaGetLastError();
+  CHD_CHECK(ok, kErrAlloc, "encoder: table allocation failed");
+  cudaMemcpyAsync(d_enc_tw, tw.data(), tw.size() * sizeof(double2), cudaMemcpyHostToDevice, stream);
+  cudaMemcpyAsync(d_galois, P->galois.data(), P->galois.size() * sizeof(int), cudaMemcpyHostToDevice, stream);
+  cudaStreamSynchronize(stream);
   return check_cuda("encoder tables");
 }
 

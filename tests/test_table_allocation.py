@@ -162,3 +162,34 @@ def test_level_constants_of_the_64_bit_path(runtime):
                 del ctx
                 n += 1
     """)
+
+
+def test_tables_of_the_encoder(runtime):
+    # built on first use; a call that had memory for one of the two tables
+    # only must not leave the next one without the other
+    runtime("""
+        p = json.load(open(os.path.join(chd.PARAM_DIR, "keyswitch_l8_a3.json")))
+        p.update(log_degree=12)
+        re, im, pt, slots = np.ones(4), np.zeros(4), np.zeros((8, 4096), np.uint32), C.c_int()
+
+        def encode(ctx):
+            chd._check(chd.lib().chd_encode(ctx.ptr, 2, 2.0 ** 30, re.ctypes.data, im.ctypes.data, 4, 0, pt.ctypes.data,
+                                            C.byref(slots)))
+
+        total, n = 1, -1
+        while n < total:
+            rt.fake_reset(-1)
+            ctx = chd.Context(json.dumps(p))
+            rt.fake_reset(n)
+            err, _ = refused(lambda: encode(ctx))
+            if n < 0:
+                total, held = rt.fake_mallocs(), rt.fake_live()
+                assert total >= 3 and err is None
+            elif n < total:
+                assert err and "failed" in err and rt.fake_launches() == 0, (n, err)
+                rt.fake_reset(-1)
+                encode(ctx)
+            assert rt.fake_launches() > 0 and rt.fake_early() == 0 and rt.fake_live() == held, n
+            ctx.close()
+            n += 1
+    """)
