@@ -641,6 +641,8 @@ Status Context64::modup(int level, const u64 *src, u64 *dst) {
   const int n = P->n;
   const NP np = P->level_np(level, m.num_aux);
   const int nq = np.q(), tot = np.total();
+  for (int i = 0; i < m.beta; i++)
+    CHD_CHECK(m.dig_e[i] - m.dig_s[i] <= 16, kErrUnsupported, "modup64: digit too large");
   std::vector<int> g(tot);
   P->gidx(np, g.data());
   ArenaScope scope(arena);

@@ -193,3 +193,19 @@ def test_tables_of_the_encoder(runtime):
             ctx.close()
             n += 1
     """)
+
+
+def test_64_bit_modup_refuses_digits_of_more_than_16_primes(runtime):
+    # as the 32-bit path does; the conversion holds 16 sources
+    runtime("""
+        p = json.load(open(os.path.join(chd.PARAM_DIR, "bootparam_40.json")))
+        q = p["main_primes"]
+        buf = np.zeros((2, 40, 65536), np.uint64)
+        for alpha, fits in ((16, True), (17, False)):
+            spec = dict(p, log_degree=16, main_primes=q[:alpha + 1], auxiliary_primes=q[20:20 + alpha], terminal_primes=[],
+                        level_config=[[alpha, 0], [alpha + 1, 0]], default_encryption_level=0, additional_base=[1, 0])
+            ctx = chd.Context64(json.dumps(spec))
+            rt.fake_reset(-1)
+            err, _ = refused(lambda: ctx.modup_raw(1, buf[0].ctypes.data, buf.ctypes.data))
+            assert (err is None) == fits and (rt.fake_launches() > 0) == fits, (alpha, err)
+    """)
