@@ -3,6 +3,8 @@
 * the reference driver library (oracle/_ref/libcheddar_ref.so, built from
   the reference's sources when the reference tree is present) exports every
   entry point oracle/refdrv.py binds;
+* the parity cases on the GPU skip only where there is no reference tree, and
+  fail where the tree is there and its driver is not;
 * the libtommath stand-in that the reference's BigInt_tommath.cpp links
   (oracle/ref_pin/shim/tommath_shim.cpp) follows libtommath's documented
   semantics on random operands, checked against Python integers: truncation
@@ -29,6 +31,20 @@ def test_reference_driver_exports():
     L = refdrv.lib()
     assert L.refx_key_index_mult() == -22222222
     assert L.refx_key_index_conj() == 11111111
+
+
+def test_parity_cases_skip_only_without_a_tree(monkeypatch, tmp_path):
+    import __graft_entry__
+    import test_gpu_refpin
+    monkeypatch.setattr(__graft_entry__, "REFERENCE", str(tmp_path))
+    monkeypatch.setattr(refdrv, "available", lambda: False)
+    with pytest.raises(pytest.skip.Exception):
+        test_gpu_refpin.need_reference()
+    (tmp_path / "src").mkdir()
+    with pytest.raises(pytest.fail.Exception):
+        test_gpu_refpin.need_reference()
+    monkeypatch.setattr(refdrv, "available", lambda: True)
+    test_gpu_refpin.need_reference()
 
 
 class MpInt(C.Structure):
