@@ -968,11 +968,12 @@ Status Context::ntt(const NP &np, uint32_t *data, bool mont, int count, size_t s
       rows.push_back(r);
     }
   return alternate_row_batches(rows, count > 1 && stride >= static_cast<size_t>(tot) * n,
-                               [&](RowBatch &rb, cudaStream_t s) { launch_ntt_fwd(rb, P->log_n, s); }, "ntt");
+                               [&](RowBatch &rb, cudaStream_t s, int beside) { launch_ntt_fwd(rb, P->log_n, s, beside); },
+                               "ntt");
 }
 
 Status Context::alternate_row_batches(const std::vector<RowDesc> &rows, bool disjoint,
-                                      const std::function<void(RowBatch &, cudaStream_t)> &launch,
+                                      const std::function<void(RowBatch &, cudaStream_t, int)> &launch,
                                       const char *what) {
   // more rows than one launch takes: the launches alternate between the
   // context stream and aux_stream (forked and joined as in fork_halves), so
@@ -984,13 +985,13 @@ Status Context::alternate_row_batches(const std::vector<RowDesc> &rows, bool dis
   const bool split = split_streams && aux_stream != nullptr && disjoint &&
                      static_cast<int>(rows.size()) > kAltRows;
   if (!split) {
-    for_row_batches(rows, [&](RowBatch &rb) { launch(rb, stream); });
+    for_row_batches(rows, [&](RowBatch &rb) { launch(rb, stream, 1); });
     return check_cuda(what);
   }
   CHD_CHECK(cudaEventRecord(ev_fork, stream) == cudaSuccess && cudaStreamWaitEvent(aux_stream, ev_fork, 0) == cudaSuccess,
             kErrCuda, "stream fork failed");
   int k = 0;
-  for_row_batches(rows, [&](RowBatch &rb) { launch(rb, (k++ & 1) ? aux_stream : stream); }, kAltRows);
+  for_row_batches(rows, [&](RowBatch &rb) { launch(rb, (k++ & 1) ? aux_stream : stream, 2); }, kAltRows);
   const bool joined =
       cudaEventRecord(ev_join, aux_stream) == cudaSuccess && cudaStreamWaitEvent(stream, ev_join, 0) == cudaSuccess;
   CHD_CHECK(joined, kErrCuda, "stream join failed");
@@ -1014,7 +1015,8 @@ Status Context::intt(const NP &np, uint32_t *data, bool mont, int count, size_t 
       rows.push_back(r);
     }
   return alternate_row_batches(rows, count > 1 && stride >= static_cast<size_t>(tot) * n,
-                               [&](RowBatch &rb, cudaStream_t s) { launch_ntt_inv(rb, P->log_n, s); }, "intt");
+                               [&](RowBatch &rb, cudaStream_t s, int beside) { launch_ntt_inv(rb, P->log_n, s, beside); },
+                               "intt");
 }
 
 Status Context::bconv(const int32_t *xt, int K, const int32_t *table, const int *dst_gidx, int M, uint32_t *out) {

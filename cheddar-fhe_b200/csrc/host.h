@@ -432,7 +432,7 @@ class Context {
   // the context stream and aux_stream when there are several batches of
   // disjoint rows
   Status alternate_row_batches(const std::vector<RowDesc> &rows, bool disjoint,
-                               const std::function<void(RowBatch &, cudaStream_t)> &launch, const char *what);
+                               const std::function<void(RowBatch &, cudaStream_t, int)> &launch, const char *what);
   Status bconv(const int32_t *xt, int K, const int32_t *table, const int *dst_gidx, int M, uint32_t *out);
   // BConv of npoly polynomials ([npoly][K][N] -> [npoly][M][N]) with the
   // host table T[m][k] (centred, Montgomery q-hat R^2): engine 0 on the CUDA

@@ -51,14 +51,16 @@ static_assert(sizeof(RowBatch) + 16 <= 32764, "row batch beyond the kernel param
 
 // Forward negacyclic NTT (bit-reversed output) of `count` limbs.
 // Column phase then row phase for log_n = 16; a single-kernel shared-memory
-// transform for log_n <= 15.  In-place allowed (dst == src).
-void launch_ntt_fwd(RowBatch &rb, int log_n, cudaStream_t s);
+// transform for log_n <= 15.  In-place allowed (dst == src).  beside: launches
+// of about this size that run at the same time on other streams, this one
+// included (they choose between one and two limbs per CTA together).
+void launch_ntt_fwd(RowBatch &rb, int log_n, cudaStream_t s, int beside = 1);
 // Row phase only / column phase only (used by fused pipelines and tests)
 void launch_ntt_fwd_cols(const RowBatch &rb, int log_n, cudaStream_t s);
-void launch_ntt_fwd_rows(RowBatch &rb, int log_n, cudaStream_t s);
+void launch_ntt_fwd_rows(RowBatch &rb, int log_n, cudaStream_t s, int beside = 1);
 // Inverse NTT (bit-reversed input); epilogue x * c0, canonical or centred
 // (kCentre).  tw must point at the inverse twiddle table.
-void launch_ntt_inv(RowBatch &rb, int log_n, cudaStream_t s);
+void launch_ntt_inv(RowBatch &rb, int log_n, cudaStream_t s, int beside = 1);
 
 // Base conversion of one job: out[m][n] = (sum_k xt[k][n] * T[m][k]) * 2^-32
 // mod p_m.  xt holds K consecutive centred limbs; destination limb m is
@@ -183,7 +185,7 @@ struct MSColBatchOf {
 using MSColBatch = MSColBatchOf<kMaxMSColJobs>;
 static_assert(sizeof(MSColBatch) + 16 <= 32764, "column-pass batch beyond the kernel parameter limit");
 void launch_modswitch_cols(const MSColBatch &b, int log_n, cudaStream_t s);
-void launch_ntt_inv_rows(RowBatch &rb, int log_n, cudaStream_t s);
+void launch_ntt_inv_rows(RowBatch &rb, int log_n, cudaStream_t s, int beside = 1);
 
 // Fused key-switching row pass (N = 2^16), see keyswitch.cu.  Modes:
 //   0 HMult:       own ModUp value a1 a2, d0 = b1 b2, d1 = b1 a2 + a1 b2

@@ -19,6 +19,7 @@
 // shared memory).  The inverse runs rows first, then columns, and fuses the
 // per-limb output constant and the optional centring into the column phase.  For N <= 2^15 the whole limb
 // fits in shared memory and one kernel runs every stage.
+#include <atomic>
 #include <type_traits>
 
 #include "arith.cuh"
@@ -255,29 +256,43 @@ void launch_ntt_fwd_cols(const RowBatch &rb, int log_n, cudaStream_t s) {
 }
 
 namespace {
+int device_sms() {
+  constexpr int kDevices = 64;
+  static std::atomic<int> cached[kDevices];
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= kDevices) dev = 0;
+  sms = cached[dev].load(std::memory_order_relaxed);
+  if (sms == 0 && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess) cached[dev] = sms;
+  return sms;
+}
+
 // Neighbouring limbs of one prime share a CTA: rb.first receives the first
-// limb of each group of one or two; returns the number of groups.  Pairs of
-// rows run at 3 CTAs per SM (80 registers), single rows at 4 (64): pairs read
-// half the twiddles (raw transforms of 32 polynomials of 24 primes 377 us
-// against 387), but half as many CTAs leave SMs idle in small launches (one
-// multiplication at level 22, 23 pairs: 102.8 us against 100.7), so pairs are
-// taken from two waves of them on.
-constexpr int kPairWaves = 2 * 3 * 148;
-int pair_rows(RowBatch &rb) {
+// limb of each group of one or two; returns the number of groups, or 0 where
+// single rows are to be taken.  Pairs of rows run at 3 CTAs per SM (80
+// registers), single rows at 4 (64): pairs read half the twiddles, but half
+// as many CTAs leave SMs idle in small launches (one multiplication at level
+// 22, 23 pairs: 102.8 us against 100.7; one launch of 48 pairs, 4 inverse
+// transforms of 24 primes: 26.6 against 25.7), so pairs are taken where they
+// fill two waves.  Two launches that alternate between streams fill them
+// together (beside = 2): 55 and 48 pairs a launch, forward and inverse
+// transforms of 32 and of 16 polynomials of 24 primes, 180 + 185 us in pairs
+// and 196 + 193 in single rows, 90 + 88 and 96 + 95.
+int pair_rows(RowBatch &rb, int beside) {
   int groups = 0;
   for (int i = 0; i < rb.count; groups++) {
     rb.first[groups] = static_cast<uint16_t>(i);
     i += i + 1 < rb.count && rb.rows[i + 1].tw == rb.rows[i].tw ? 2 : 1;
   }
   rb.first[groups] = static_cast<uint16_t>(rb.count);
-  return groups;
+  if (groups == rb.count) return 0;
+  return groups * kLimbRows * beside < 2 * 3 * device_sms() ? 0 : groups;
 }
 }  // namespace
 
-void launch_ntt_fwd_rows(RowBatch &rb, int log_n, cudaStream_t s) {
+void launch_ntt_fwd_rows(RowBatch &rb, int log_n, cudaStream_t s, int beside) {
   if (rb.count <= 0) return;
-  const int groups = pair_rows(rb);
-  if (groups == rb.count || groups * kLimbRows < kPairWaves)
+  const int groups = pair_rows(rb, beside);
+  if (!groups)
     with_rows(rb, [&](const auto &b) {
       launch_dependent(k_fwd_rows16<1, 4, std::decay_t<decltype(b)>>, dim3(kLimbRows, b.count), kRowThreads, 0, s, b);
     });
@@ -285,11 +300,11 @@ void launch_ntt_fwd_rows(RowBatch &rb, int log_n, cudaStream_t s) {
     launch_dependent(k_fwd_rows16<2, 3, RowBatch>, dim3(kLimbRows, groups), kRowThreads, 0, s, rb);
 }
 
-void launch_ntt_fwd(RowBatch &rb, int log_n, cudaStream_t s) {
+void launch_ntt_fwd(RowBatch &rb, int log_n, cudaStream_t s, int beside) {
   if (rb.count <= 0) return;
   if (log_n == 16) {
     launch_ntt_fwd_cols(rb, log_n, s);
-    launch_ntt_fwd_rows(rb, log_n, s);
+    launch_ntt_fwd_rows(rb, log_n, s, beside);
   } else {
     size_t smem = sizeof(uint32_t) << log_n;
     cudaFuncSetAttribute(k_small<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024);
@@ -297,10 +312,10 @@ void launch_ntt_fwd(RowBatch &rb, int log_n, cudaStream_t s) {
   }
 }
 
-void launch_ntt_inv_rows(RowBatch &rb, int log_n, cudaStream_t s) {
+void launch_ntt_inv_rows(RowBatch &rb, int log_n, cudaStream_t s, int beside) {
   if (rb.count <= 0) return;
-  const int groups = pair_rows(rb);
-  if (groups == rb.count || groups * kLimbRows < kPairWaves)
+  const int groups = pair_rows(rb, beside);
+  if (!groups)
     with_rows(rb, [&](const auto &b) {
       launch_dependent(k_inv_rows16<1, 4, std::decay_t<decltype(b)>>, dim3(kLimbRows, b.count), kRowThreads, 0, s, b);
     });
@@ -308,10 +323,10 @@ void launch_ntt_inv_rows(RowBatch &rb, int log_n, cudaStream_t s) {
     launch_dependent(k_inv_rows16<2, 3, RowBatch>, dim3(kLimbRows, groups), kRowThreads, 0, s, rb);
 }
 
-void launch_ntt_inv(RowBatch &rb, int log_n, cudaStream_t s) {
+void launch_ntt_inv(RowBatch &rb, int log_n, cudaStream_t s, int beside) {
   if (rb.count <= 0) return;
   if (log_n == 16) {
-    launch_ntt_inv_rows(rb, log_n, s);
+    launch_ntt_inv_rows(rb, log_n, s, beside);
     with_rows(rb, [&](const auto &b) {
       launch_dependent(k_inv_cols16<std::decay_t<decltype(b)>>, dim3(kRowLen / kColThreads, b.count), kColThreads, 0, s,
                        b);
