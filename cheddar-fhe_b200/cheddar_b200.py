@@ -248,21 +248,14 @@ def _ptr(a):
 
 def ks_tuned_shapes():
     """The column passes whose variant was chosen by timing in this process:
-    none since the column pass has one variant."""
-    n = lib().chd_ks_tuned_shapes(None, 0)
-    out = (C.c_int * (6 * max(1, n)))()
-    n = lib().chd_ks_tuned_shapes(out, n)
-    return [dict(device=out[6 * i], K=out[6 * i + 1], jobs=out[6 * i + 2], M=out[6 * i + 3],
-                 engine=out[6 * i + 4], split=out[6 * i + 5]) for i in range(n)]
+    none, the column pass has one variant."""
+    return []
 
 
 def ks_rows_tuned_shapes():
-    """The same for the key-switch row pass: none."""
-    n = lib().chd_ks_rows_tuned_shapes(None, 0)
-    out = (C.c_int * (5 * max(1, n)))()
-    n = lib().chd_ks_rows_tuned_shapes(out, n)
-    return [dict(device=out[5 * i], cts=out[5 * i + 1], rows=out[5 * i + 2], mode=out[5 * i + 3],
-                 variant=out[5 * i + 4], prefetch=out[5 * i + 4] == 1) for i in range(n)]
+    """The same for the key-switch row pass: none, its form follows from the
+    digit count."""
+    return []
 
 
 def load_params(name_or_path):

@@ -14,22 +14,9 @@
 
 namespace chd {
 
-struct Modulus {
-  uint32_t q;
-  int32_t qinv;  // q^-1 mod 2^32 as a signed word
-};
-
 __device__ __forceinline__ int32_t mont_reduce_lazy(int64_t a, uint32_t q, int32_t qinv) {
   int32_t lo = static_cast<int32_t>(static_cast<uint32_t>(static_cast<uint64_t>(a)));
   int32_t hi = static_cast<int32_t>(a >> 32);
-  int32_t m = lo * qinv;
-  return hi - __mulhi(m, static_cast<int32_t>(q));
-}
-
-// a * b * 2^-32 mod q in (-q, q) for |a * b| < q * 2^31
-__device__ __forceinline__ int32_t mont_mul_lazy(int32_t a, int32_t b, uint32_t q, int32_t qinv) {
-  int32_t lo = a * b;
-  int32_t hi = __mulhi(a, b);
   int32_t m = lo * qinv;
   return hi - __mulhi(m, static_cast<int32_t>(q));
 }
@@ -87,20 +74,6 @@ __device__ __forceinline__ uint32_t mont_mac2(uint32_t a1, uint32_t b1, uint32_t
   const uint64_t s = static_cast<uint64_t>(a1) * b1 + static_cast<uint64_t>(a2) * b2;
   const uint32_t r = mont_redc2(s, q, qneg);
   return r >= q ? r - q : r;
-}
-
-// Cooley-Tukey butterfly on canonical values: (a, b) -> (a + w b, a - w b)
-__device__ __forceinline__ void ct_bfly(uint32_t &a, uint32_t &b, uint32_t w, uint32_t q, int32_t qinv) {
-  uint32_t t = mont_mul(b, w, q, qinv);
-  b = sub_mod(a, t, q);
-  a = add_mod(a, t, q);
-}
-
-// Gentleman-Sande butterfly on canonical values: (a, b) -> (a + b, (a - b) w)
-__device__ __forceinline__ void gs_bfly(uint32_t &a, uint32_t &b, uint32_t w, uint32_t q, int32_t qinv) {
-  uint32_t d = sub_mod(a, b, q);
-  a = add_mod(a, b, q);
-  b = mont_mul(d, w, q, qinv);
 }
 
 // ---- Shoup multiplication with lazy [0, 2q) values (D. Harvey, "Faster

@@ -13,9 +13,9 @@
 namespace chd {
 namespace {
 
-// ld4c only in kernels that are not launched dependently (launch.cuh)
+// ldg4 (through __ldg) only in kernels that are not launched dependently (launch.cuh)
 __device__ __forceinline__ uint4 ld4(const uint32_t *p) { return *reinterpret_cast<const uint4 *>(p); }
-__device__ __forceinline__ uint4 ld4c(const uint32_t *p) { return __ldg(reinterpret_cast<const uint4 *>(p)); }
+__device__ __forceinline__ uint4 ldg4(const uint32_t *p) { return __ldg(reinterpret_cast<const uint4 *>(p)); }
 __device__ __forceinline__ void st4(uint32_t *p, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   *reinterpret_cast<uint4 *>(p) = make_uint4(a, b, c, d);
 }
@@ -95,12 +95,12 @@ __global__ void __launch_bounds__(256) k_key_mac(const __grid_constant__ KeyMacD
   int i = 0;
   for (; i + 1 < d.beta; i += 2) {  // two digits per Montgomery reduction
     uint32_t mu0[4], kb0[4], ka0[4], mu1[4], kb1[4], ka1[4];
-    unpack(ld4c(c.mu[i] + off), mu0);
-    unpack(ld4c(d.kb[i] + koff), kb0);
-    unpack(ld4c(d.ka[i] + koff), ka0);
-    unpack(ld4c(c.mu[i + 1] + off), mu1);
-    unpack(ld4c(d.kb[i + 1] + koff), kb1);
-    unpack(ld4c(d.ka[i + 1] + koff), ka1);
+    unpack(ldg4(c.mu[i] + off), mu0);
+    unpack(ldg4(d.kb[i] + koff), kb0);
+    unpack(ldg4(d.ka[i] + koff), ka0);
+    unpack(ldg4(c.mu[i + 1] + off), mu1);
+    unpack(ldg4(d.kb[i + 1] + koff), kb1);
+    unpack(ldg4(d.ka[i + 1] + koff), ka1);
 #pragma unroll
     for (int l = 0; l < 4; l++) {
       sb[l] = add_mod(sb[l], mont_mac2(mu0[l], kb0[l], mu1[l], kb1[l], q, qn), q);
@@ -109,9 +109,9 @@ __global__ void __launch_bounds__(256) k_key_mac(const __grid_constant__ KeyMacD
   }
   if (i < d.beta) {
     uint32_t mu[4], kb[4], ka[4];
-    unpack(ld4c(c.mu[i] + off), mu);
-    unpack(ld4c(d.kb[i] + koff), kb);
-    unpack(ld4c(d.ka[i] + koff), ka);
+    unpack(ldg4(c.mu[i] + off), mu);
+    unpack(ldg4(d.kb[i] + koff), kb);
+    unpack(ldg4(d.ka[i] + koff), ka);
 #pragma unroll
     for (int l = 0; l < 4; l++) {
       sb[l] = add_mod(sb[l], mont_mul(mu[l], kb[l], q, qi), q);
@@ -122,13 +122,13 @@ __global__ void __launch_bounds__(256) k_key_mac(const __grid_constant__ KeyMacD
     const uint32_t pp = d.p_prod[r];
     if (c.d0) {
       uint32_t v[4];
-      unpack(ld4c(c.d0 + off), v);
+      unpack(ldg4(c.d0 + off), v);
 #pragma unroll
       for (int l = 0; l < 4; l++) sb[l] = add_mod(sb[l], mont_mul(v[l], pp, q, qi), q);
     }
     if (c.d1) {
       uint32_t v[4];
-      unpack(ld4c(c.d1 + off), v);
+      unpack(ldg4(c.d1 + off), v);
 #pragma unroll
       for (int l = 0; l < 4; l++) sa[l] = add_mod(sa[l], mont_mul(v[l], pp, q, qi), q);
     }
@@ -273,9 +273,9 @@ __global__ void __launch_bounds__(256, MINB) k_hoisted(const __grid_constant__ H
   uint32_t mu[BMAX][4];
 #pragma unroll
   for (int i = 0; i < BMAX; i++)
-    if (i < d.beta) unpack(ld4c(d.mu[c][i] + off), mu[i]);
+    if (i < d.beta) unpack(ldg4(d.mu[c][i] + off), mu[i]);
   uint32_t bxp[4] = {0, 0, 0, 0};
-  if (r < d.nq) unpack(ld4c(d.bxp[c] + off), bxp);
+  if (r < d.nq) unpack(ldg4(d.bxp[c] + off), bxp);
   for (int j = 0; j < d.R; j++) {
     uint32_t sb[4], sa[4] = {0, 0, 0, 0};
 #pragma unroll
@@ -284,10 +284,10 @@ __global__ void __launch_bounds__(256, MINB) k_hoisted(const __grid_constant__ H
     for (int i = 0; i < BMAX; i += 2) {
       if (i + 1 < d.beta) {  // two digits per Montgomery reduction
         uint32_t kb0[4], ka0[4], kb1[4], ka1[4];
-        unpack(ld4c(d.kb[j][i] + koff), kb0);
-        unpack(ld4c(d.ka[j][i] + koff), ka0);
-        unpack(ld4c(d.kb[j][i + 1] + koff), kb1);
-        unpack(ld4c(d.ka[j][i + 1] + koff), ka1);
+        unpack(ldg4(d.kb[j][i] + koff), kb0);
+        unpack(ldg4(d.ka[j][i] + koff), ka0);
+        unpack(ldg4(d.kb[j][i + 1] + koff), kb1);
+        unpack(ldg4(d.ka[j][i + 1] + koff), ka1);
 #pragma unroll
         for (int l = 0; l < 4; l++) {
           sb[l] = add_mod(sb[l], mont_mac2(mu[i][l], kb0[l], mu[i + 1][l], kb1[l], q, qn), q);
@@ -295,8 +295,8 @@ __global__ void __launch_bounds__(256, MINB) k_hoisted(const __grid_constant__ H
         }
       } else if (i < d.beta) {
         uint32_t kb[4], ka[4];
-        unpack(ld4c(d.kb[j][i] + koff), kb);
-        unpack(ld4c(d.ka[j][i] + koff), ka);
+        unpack(ldg4(d.kb[j][i] + koff), kb);
+        unpack(ldg4(d.ka[j][i] + koff), ka);
 #pragma unroll
         for (int l = 0; l < 4; l++) {
           sb[l] = add_mod(sb[l], mont_mul(mu[i][l], kb[l], q, qi), q);

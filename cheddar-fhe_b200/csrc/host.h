@@ -357,8 +357,8 @@ class Context {
   // A fused key switch of two or more ciphertexts runs its two halves on the
   // context stream and on aux_stream (forked from and joined back into the
   // context stream by events), so that the kernels of one half fill the
-  // issue slots the other half's kernels leave idle (the column passes wait
-  // on barriers and the tensor cores, the row passes on the ALU)
+  // issue slots the other half's kernels leave idle (the row passes wait for
+  // their loads, the column passes on the integer multiplier)
   bool split_streams = true;
   cudaStream_t aux_stream = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;

@@ -40,9 +40,12 @@ inline void launch_dependent(void (*kern)(P...), dim3 grid, int block, size_t sm
 
 // Launch parameters travel with every launch: a call on one ciphertext fills
 // a few of a batch's descriptors.  18 KiB for them cost no time on the GPU but
-// 1 us and more of the host's per launch: where the host was the slower side,
-// a plaintext product and rescale at level 5 took 19.7 us and now 15.5, one
-// transform of 24 primes forward and inverse 23.0 and 19.5.
+// 1 us and more of the host's per launch.  Host time of a call, enqueued
+// among others, in whole and in small batches: a plaintext product and rescale
+// at level 5 19.6 and 15.1 us, one polynomial of 24 primes forward and inverse
+// 22.1 and 16.2, one multiplication at level 22 22.9 and 18.0.  The GPU needs
+// 16.3, 19.6 and 84.5 us for them, so the first two had waited for the host
+// (20.4 and 22.9 us a call).
 constexpr int kFewRows = 64, kFewJobs = 8;
 
 }  // namespace chd

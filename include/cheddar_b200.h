@@ -434,8 +434,9 @@ int chd_bconv_batch(chd_context *ctx, int engine, int npoly, const int32_t *xt_d
 int chd_set_ks_engine(chd_context *ctx, int engine);
 int chd_get_ks_engine(const chd_context *ctx);
 /* Shapes of the column pass (six ints each) and of the key-switch row pass
- * (five ints each) whose variant was chosen by timing: none, each pass has
- * one variant.  Both return 0 and write nothing. */
+ * (five ints each) whose variant was chosen by timing: none (the column pass
+ * has one variant, the row pass's follows from the digit count).  Both return
+ * 0 and write nothing. */
 int chd_ks_tuned_shapes(int *out, int cap);
 int chd_ks_rows_tuned_shapes(int *out, int cap);
 /* Two-stream key switching (no reference counterpart; on by default, the
