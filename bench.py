@@ -18,8 +18,8 @@ Reported (one JSON line on rank 0):
   cpu_baseline  the CPU oracle's HMult on the host cores (bounded sample)
   bootstrap  full-slot bootstrapping throughput at N = 2^16 (bootstraps/s;
              decoded precision with real keys: tests/boot_precision_n16.py)
-  ks_engines  the same step under each chd_set_ks_engine value (--ks-engine
-             picks the measured one; one column pass serves them all)
+  eager_vs_graph  the step as one call per pair, eager, and as one batched
+             call replayed as a CUDA graph
   bconv_engines  base conversion on CUDA cores vs tcgen05 tensor cores
   ntt        forward + inverse NTT round trip, 24 primes, HBM fraction
 `--impl reference` times the CPU implementation of the path (the oracle;
@@ -167,7 +167,9 @@ def main():
     ap.add_argument("--no-reference-gpu", action="store_true",
                     help="skip timing the reference's own sm_100a build on the same workloads")
     ap.add_argument("--ks-engine", default="auto", choices=["cuda", "tensor", "tensor_wide", "auto"],
-                    help="base conversion inside the ModUp / ModDown column passes of the measured path")
+                    help="chd_set_ks_engine value of the measured path: one column pass serves all of them; "
+                         "auto also times the register variants of the hoisted rotations and the plaintext "
+                         "accumulation on their first launch")
     ap.add_argument("--hmult-only", action="store_true",
                     help="profiling aid: measure only the HMult step (value, e2e, roofline) and print its line")
     args = ap.parse_args()
@@ -261,7 +263,7 @@ def main():
     # dominant kernel and its roofline ----
     ctx.stream_split = False
     for _ in range(3):
-        step()  # the one-stream launch shapes tuned outside the timed spans
+        step()  # outside the timed spans
     ctx.stage_timing(True)
     for _ in range(args.steps):
         step()
@@ -270,14 +272,12 @@ def main():
     ctx.stream_split = True
     roof = roofline_from_stages(ctx, lvl, B, stages, args.steps)
 
-    ks_cmp = bconv_cmp = ntt_cmp = hoist_mixed = w64 = boot = split_cmp = None
+    graph_cmp = bconv_cmp = ntt_cmp = hoist_mixed = w64 = boot = split_cmp = None
     if not args.hmult_only:
         # ---- the same step with the key switch on one stream ----
         split_cmp = stream_split_cmp(ctx, step, stream, args.steps)
-        # ---- the same step with each column-pass engine ----
-        ks_cmp = ks_engines(ctx, chd, step, stream, args.steps, B)
-        ks_cmp["plain_vs_tensor_batched"] = plain_vs_batched_hmult(ctx, chd, key, a_cts, b_cts, outs, stream,
-                                                                   args.steps)
+        # ---- one call per pair against one graph-replayed batch ----
+        graph_cmp = eager_vs_graph_hmult(ctx, key, a_cts, b_cts, outs, stream, args.steps)
 
         # ---- base conversion as a dense contraction: CUDA cores vs tensor cores ----
         bconv_cmp = bconv_engines(ctx, chd, stream)
@@ -305,21 +305,10 @@ def main():
                    "l2": "inputs larger than L2 (batch x 24 MB + 48 MB key)",
                    "parallelism": f"replicas x{world}"},
         "e2e": e2e, "roofline": roof, "clocks": sampler.summary(), "ks_engine": args.ks_engine,
-        "ks_engines": ks_cmp, "bconv_engines": bconv_cmp, "ntt": ntt_cmp,
+        "eager_vs_graph": graph_cmp, "bconv_engines": bconv_cmp, "ntt": ntt_cmp,
         "bootstrap": boot, "hoisted_and_mixed": hoist_mixed, "w64": w64, "stream_split": split_cmp,
         "gpu_launches": launches,
     }
-    # column and row passes whose variant was chosen by timing: none, each
-    # has one variant (the keys stay for readers of earlier lines)
-    line["config"]["autotuned_column_passes"] = [
-        f"K{t['K']} jobs{t['jobs']} M{t['M']}: "
-        f"{({0: 'cuda_core', 1: 'tensor_core', 3: 'tensor_core_wide', 4: 'tensor_core_wide_128regs'}).get(t['engine'], t['engine'])}"
-        f"/split{t['split']}"
-        for t in chd.ks_tuned_shapes()]
-    line["config"]["autotuned_row_passes"] = [
-        f"cts{t['cts']} rows{t['rows']} mode{t['mode']}: "
-        f"{({0: 'in_place_loads', 1: 'prefetch', 2: 'in_place_loads_4ctas'}).get(t['variant'], t['variant'])}"
-        for t in chd.ks_rows_tuned_shapes()]
     if rank == 0 and world == 1 and not args.no_reference_gpu and not args.hmult_only:
         ref = reference_gpu_run(args)
         try:
@@ -531,46 +520,6 @@ def ks_engine_id(chd, args):
             "auto": chd.BCONV_AUTO}[args.ks_engine]
 
 
-def ks_engines(ctx, chd, step, stream, steps, B):
-    """The HMult step under each chd_set_ks_engine value: one column pass
-    serves them all, so the times agree within noise.  The one-stream
-    pipeline, so that the stage events time each column pass alone."""
-    import torch
-    old = ctx.ks_engine
-    ctx.stream_split = False
-    out = {}
-    for name, e in (("cuda_core", chd.BCONV_CUDA_CORE), ("tensor_core", chd.BCONV_TENSOR_CORE),
-                    ("tensor_core_wide", chd.BCONV_TENSOR_CORE_WIDE), ("auto", chd.BCONV_AUTO)):
-        ctx.ks_engine = e
-        for _ in range(3):
-            step()
-        torch.cuda.synchronize()
-        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        e0.record(stream)
-        for _ in range(steps):
-            step()
-        e1.record(stream)
-        torch.cuda.synchronize()
-        ms = e0.elapsed_time(e1)
-        ctx.stage_timing(True)
-        for _ in range(steps):
-            step()
-        st = ctx.stage_times()
-        ctx.stage_timing(False)
-        out[name] = {"hmult_per_s": B * steps / (ms / 1e3), "ms_per_step": ms / steps,
-                     "modup_cols_ms": st["modup_cols"][0] / steps, "moddown_cols_ms": st["moddown_cols"][0] / steps}
-    ctx.ks_engine = old
-    ctx.stream_split = True
-    out["speedup_tensor_vs_cuda_core"] = out["tensor_core"]["hmult_per_s"] / out["cuda_core"]["hmult_per_s"]
-    out["speedup_tensor_wide_vs_cuda_core"] = (out["tensor_core_wide"]["hmult_per_s"] /
-                                               out["cuda_core"]["hmult_per_s"])
-    cols = {k: out[k]["modup_cols_ms"] + out[k]["moddown_cols_ms"] for k in ("cuda_core", "tensor_core",
-                                                                           "tensor_core_wide")}
-    out["column_pass_speedup"] = cols["cuda_core"] / cols["tensor_core"]
-    out["column_pass_speedup_wide"] = cols["cuda_core"] / cols["tensor_core_wide"]
-    return out
-
-
 def stream_split_cmp(ctx, step, stream, steps):
     """The measured step with the fused key switch split over two streams
     (the default: halves of the batch on the context stream and on the
@@ -596,13 +545,10 @@ def stream_split_cmp(ctx, step, stream, steps):
     return res
 
 
-def plain_vs_batched_hmult(ctx, chd, key, a_cts, b_cts, outs, stream, steps):
-    """The two forms the design targets compare, same B pairs:
-    plain = one HMult call per pair, CUDA-core column passes, eager launches;
-    tensor-core batched = one HMultBatch over all B on the tensor-core
-    engine, captured once as a CUDA graph and replayed."""
+def eager_vs_graph_hmult(ctx, key, a_cts, b_cts, outs, stream, steps):
+    """The same B pairs as one HMult call per pair with eager launches, and as
+    one HMultBatch over all B captured once as a CUDA graph and replayed."""
     import torch
-    old = ctx.ks_engine
     B = len(a_cts)
 
     def timed(fn):
@@ -618,25 +564,21 @@ def plain_vs_batched_hmult(ctx, chd, key, a_cts, b_cts, outs, stream, steps):
         torch.cuda.synchronize()
         return e0.elapsed_time(e1) / steps
 
-    ctx.ks_engine = chd.BCONV_CUDA_CORE
-
-    def plain():
+    def one_by_one():
         for i in range(B):
             ctx.HMult(a_cts[i], b_cts[i], key, rescale=True, res=outs[i])
 
-    ms_plain = timed(plain)
-    ctx.ks_engine = chd.BCONV_TENSOR_CORE
+    ms_one = timed(one_by_one)
     ctx.HMultBatch(a_cts, b_cts, key, rescale=True, res_list=outs)
     ctx.synchronize()
     ctx.graph_begin()
     ctx.HMultBatch(a_cts, b_cts, key, rescale=True, res_list=outs)
     graph = ctx.graph_end()
-    ms_tc = timed(graph.launch)
+    ms_graph = timed(graph.launch)
     del graph
-    ctx.ks_engine = old
-    return {"plain_cuda_core_one_by_one": {"hmult_per_s": B / (ms_plain / 1e3), "ms_per_step": ms_plain},
-            "tensor_core_batched_graph": {"hmult_per_s": B / (ms_tc / 1e3), "ms_per_step": ms_tc},
-            "speedup": ms_plain / ms_tc}
+    return {"one_by_one_eager": {"hmult_per_s": B / (ms_one / 1e3), "ms_per_step": ms_one},
+            "batched_graph": {"hmult_per_s": B / (ms_graph / 1e3), "ms_per_step": ms_graph},
+            "speedup": ms_one / ms_graph}
 
 
 NTT_PARAM_FILE = "ntt_bootparam30_p24.json"
@@ -946,7 +888,7 @@ def w64_bench(chd, stream, steps=20, warmup=3):
     g.set_stream(None)
     return {"workload": f"64-bit word path: HMult+relin+rescale at the top level of {W64_PARAM_FILE}",
             "ms_per_hmult": ms, "hmult_per_s": 1e3 / ms, "steps": steps,
-            "kernels": "unfused: two-pass NTT, exact 128-bit base conversion, element-wise"}
+            "kernels": "unfused: two-pass NTT, exact base conversion, element-wise"}
 
 
 def _peaks():
@@ -1161,30 +1103,6 @@ def boot_bench(chd, args, stream, dist, profile=False):
     ctx.synchronize()
     torch.cuda.synchronize()
     ms_single = es0.elapsed_time(es1)
-    # the plain form: one ciphertext per call on the CUDA-core engine
-    main_engine = ctx.ks_engine
-    ctx.ks_engine = chd.BCONV_CUDA_CORE
-    step_single()
-    ctx.synchronize()
-    es0.record(stream)
-    for _ in range(steps):
-        step_single()
-    es1.record(stream)
-    ctx.synchronize()
-    torch.cuda.synchronize()
-    ms_plain = es0.elapsed_time(es1)
-    # one ciphertext per call with the autotuned engine
-    ctx.ks_engine = chd.BCONV_AUTO
-    step_single()
-    ctx.synchronize()
-    es0.record(stream)
-    for _ in range(steps):
-        step_single()
-    es1.record(stream)
-    ctx.synchronize()
-    torch.cuda.synchronize()
-    ms_single_auto = es0.elapsed_time(es1)
-    ctx.ks_engine = main_engine
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     barrier(dist)
     torch.cuda.synchronize()
@@ -1242,11 +1160,11 @@ def boot_bench(chd, args, stream, dist, profile=False):
     ctx.synchronize()
     torch.cuda.synchronize()
     ms_mk = e2.elapsed_time(e3)
-    # the same bootstraps with each column-pass engine
-    engines = {}
+    # the same eager batch with the hoisted rotations' and plaintext
+    # accumulations' register variants fixed, and chosen by timing
+    variants = {}
     main_engine = ctx.ks_engine
-    for name, e in (("cuda_core", chd.BCONV_CUDA_CORE), ("tensor_core", chd.BCONV_TENSOR_CORE),
-                    ("tensor_core_wide", chd.BCONV_TENSOR_CORE_WIDE), ("auto", chd.BCONV_AUTO)):
+    for name, e in (("fixed", chd.BCONV_CUDA_CORE), ("timed", chd.BCONV_AUTO)):
         ctx.ks_engine = e
         step()
         ctx.synchronize()
@@ -1256,13 +1174,8 @@ def boot_bench(chd, args, stream, dist, profile=False):
         e3.record(stream)
         ctx.synchronize()
         torch.cuda.synchronize()
-        t = e2.elapsed_time(e3)
-        engines[name] = {"ms_per_boot": t / (B * steps), "bootstraps_per_s": B * steps / (t / 1e3)}
+        variants[name + "_ms_per_boot"] = e2.elapsed_time(e3) / (B * steps)
     ctx.ks_engine = main_engine
-    engines["speedup_tensor_vs_cuda_core"] = (engines["tensor_core"]["bootstraps_per_s"] /
-                                              engines["cuda_core"]["bootstraps_per_s"])
-    engines["speedup_tensor_wide_vs_cuda_core"] = (engines["tensor_core_wide"]["bootstraps_per_s"] /
-                                                   engines["cuda_core"]["bootstraps_per_s"])
     try:
         data_l, const_l = boot_trace_limbs(ctx, bc, params)
         hbm = _peaks().get("hbm_gbs", 6650.0)
@@ -1284,18 +1197,17 @@ def boot_bench(chd, args, stream, dist, profile=False):
            "value": job_throughput(world, B, steps, ms_graph),
            "eager": {"bootstraps_per_s": world * B * steps / (ms / 1e3), "ms_per_boot": ms / (B * steps)},
            "one_by_one_eager": {"bootstraps_per_s": world * B * steps / (ms_single / 1e3),
-                                "ms_per_boot": ms_single / (B * steps),
-                                "ms_per_boot_auto_engine": ms_single_auto / (B * steps)},
-           "plain_vs_tensor_batched": {
-               "plain_cuda_core_one_by_one_ms_per_boot": ms_plain / (B * steps),
-               "tensor_core_batched_graph_ms_per_boot": ms_graph / (B * steps),
-               "speedup": ms_plain / ms_graph},
+                                "ms_per_boot": ms_single / (B * steps)},
+           "eager_vs_graph": {
+               "one_by_one_eager_ms_per_boot": ms_single / (B * steps),
+               "batched_graph_ms_per_boot": ms_graph / (B * steps),
+               "speedup": ms_single / ms_graph},
            "stream_split": {"one_stream_ms_per_boot": ms_graph_one / (B * steps),
                             "two_streams_ms_per_boot": ms_graph / (B * steps), "speedup": ms_graph_one / ms_graph},
            "min_ks": {"ms_per_boot": ms_mk / (B * steps), "bootstraps_per_s": B * steps / (ms_mk / 1e3),
                       "rotation_keys": len(bc.rotations(min_ks=True))},
            "unit": "bootstraps/s", "ms_per_boot": ms_graph / (B * steps), "batch_per_gpu": B, "steps": steps,
-           "ks_engine": args.ks_engine, "ks_engines": engines,
+           "ks_engine": args.ks_engine, "register_variants": variants,
            "warmup": 2, "params": f"{BOOT_PARAM_FILE}: the reference's own 40-bit bootstrapping parameter file "
                                   "(4 terminal + 43 main primes, max level 28, alpha=12, sparse-secret "
                                   "encapsulation), 4 CtS + 3 StC levels, EvalMod deg-30 Chebyshev cosine + 3 "
