@@ -150,15 +150,16 @@ __device__ __forceinline__ void inner_product(const KSRowsCt &c, const KSRowsLev
   }
 }
 
-// What bounds it: integer issue (61 % of cycles, the multiplier 64 % busy) and
+// What bounds it: integer issue (64 % of cycles, the multiplier 68 % busy) and
 // the latency of its loads, so occupancy decides.  Each digit's transformed
 // row waits in shared memory and the inner product runs over four
 // coefficients at a time, so that 64 registers suffice and four CTAs share an
-// SM.  8 multiplications at level 22, one stream: 198 us; with 64-bit
-// accumulators of the whole row in registers (128, two CTAs) 235, with 32-bit
-// ones (80 and spilled, three CTAs) 224; the 128 x 512 form before it 218
-// with three stages fewer.  Two digits per transform (sharing twiddles, 80
-// registers, three CTAs) 227; L2 prefetch of the key rows no gain.
+// SM.  8 multiplications at level 22, one stream: 186 us.  Beside a form of it
+// that took 198: with 64-bit accumulators of the whole row in registers (128,
+// two CTAs) 235, with 32-bit ones (80 and spilled, three CTAs) 224; the 128 x
+// 512 form before it 218 with three stages fewer.  Two digits per transform
+// (sharing twiddles, 80 registers, three CTAs) 227; L2 prefetch of the key
+// rows no gain.
 //
 // More than four digits (GROUPED) go through two row buffers in groups of two,
 // the sums between groups in two more: 64 KiB and three CTAs whatever the

@@ -79,7 +79,7 @@ __device__ __forceinline__ uint32_t join(int d0, int d1, int d2, int d3, uint32_
 // to 96 / 74 us; one step tighter spills and gives 94 / 76 us.
 //
 // Measured, 8 multiplications at level 22 on one stream: ModUp (24 jobs of
-// 8 sources and 24 targets) 85 us, ModDown + Rescale (16 jobs of 9 and 23)
+// 8 sources and 24 targets) 82 us, ModDown + Rescale (16 jobs of 9 and 23)
 // 68 us; the 128 x 512 tcgen05 pass before it took 172 and 141 us.
 template <int KR, int MINB, class B>
 __global__ void __launch_bounds__(32 * kColWarps, MINB) k_modswitch_cols(const __grid_constant__ B b) {
