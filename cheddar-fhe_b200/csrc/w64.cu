@@ -561,12 +561,18 @@ const LevelMS64 *Context64::lms(int level) {
     auto m = std::make_unique<LevelMS64>();
     build_level_ms64(*P, level, m.get());
     m->d_mod_up2.assign(m->mod_up2.size(), nullptr);
-    bool ok = true;
-    for (size_t i = 0; i < m->mod_up2.size(); i++) ok = ok && upload(m->mod_up2[i], stream, &m->d_mod_up2[i]);
-    ok = ok && upload(m->mod_down2, stream, &m->d_mod_down2) && upload(m->rs2, stream, &m->d_rs2) &&
-         upload(m->mdr2, stream, &m->d_mdr2);
-    // complete before use: k64_bconv reads its table ahead of the kernels before it
-    if (cudaStreamSynchronize(stream) != cudaSuccess || !ok) {
+    // on a stream of their own, as the context's may be capturing a graph, and
+    // complete before use: k64_bconv reads its table ahead of the kernels
+    // before it
+    cudaStream_t s = nullptr;
+    bool ok = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess;
+    for (size_t i = 0; i < m->mod_up2.size(); i++) ok = ok && upload(m->mod_up2[i], s, &m->d_mod_up2[i]);
+    ok = ok && upload(m->mod_down2, s, &m->d_mod_down2) && upload(m->rs2, s, &m->d_rs2) && upload(m->mdr2, s, &m->d_mdr2);
+    if (s) {
+      ok = cudaStreamSynchronize(s) == cudaSuccess && ok;
+      cudaStreamDestroy(s);
+    }
+    if (!ok) {
       cudaGetLastError();
       set_error("64-bit level constants: device allocation or copy failed");
       return nullptr;

@@ -3,7 +3,8 @@ machines without a GPU: a subprocess preloads it, device memory is host
 memory, kernels do not run.  It refuses the n-th allocation, counts kernel
 launches and keeps their grids, and counts launches that come after a copy
 from pageable host memory (which may return early, and which other streams do
-not wait for) and before a synchronisation."""
+not wait for) and before a synchronisation.  On the stream that a test names as
+capturing, copies are recorded only and a synchronisation fails."""
 import os
 import subprocess
 import sys
@@ -35,6 +36,8 @@ long fake_early(void) { return early; }
 int fake_last(void) { return last; }
 void fake_reset(long n) { mallocs = launches = early = 0; fail_at = n; }
 static cudaError_t ok(void) { return cudaSuccess; }
+static cudaStream_t capturing;
+void fake_capture(void *s) { capturing = s; }
 cudaError_t cudaMalloc(void **p, size_t n) {
   if (mallocs++ == fail_at) return last = cudaErrorMemoryAllocation;
   *p = calloc(1, n);
@@ -48,7 +51,7 @@ cudaError_t cudaMemcpy(void *d, const void *s, size_t n, enum cudaMemcpyKind k) 
   return ok();
 }
 cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, enum cudaMemcpyKind k, cudaStream_t t) {
-  memmove(d, s, n);
+  if (!capturing || t != capturing) memmove(d, s, n);
   return ok();
 }
 cudaError_t cudaMemset(void *d, int v, size_t n) { memset(d, v, n); return ok(); }
@@ -59,7 +62,9 @@ cudaError_t cudaDeviceGetAttribute(int *v, enum cudaDeviceAttr a, int d) { *v = 
 cudaError_t cudaDeviceSynchronize(void) { copying = 0; return ok(); }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned f) { *s = (cudaStream_t)malloc(1); return ok(); }
 cudaError_t cudaStreamDestroy(cudaStream_t s) { free(s); return ok(); }
-cudaError_t cudaStreamSynchronize(cudaStream_t s) { return ok(); }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) {
+  return capturing && s == capturing ? (last = cudaErrorStreamCaptureUnsupported) : ok();
+}
 cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned f) { return ok(); }
 cudaError_t cudaStreamIsCapturing(cudaStream_t s, enum cudaStreamCaptureStatus *c) { *c = 0; return ok(); }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned f) { *e = (cudaEvent_t)malloc(1); return ok(); }
@@ -87,6 +92,7 @@ for f in ("fake_mallocs", "fake_live", "fake_launches", "fake_early"):
     getattr(rt, f).restype = C.c_long
 rt.fake_reset.argtypes = [C.c_long]
 rt.fake_grid.argtypes = [C.c_long, C.c_int]
+rt.fake_capture.argtypes = [C.c_void_p]
 
 def refused(make):
     try:

@@ -62,6 +62,25 @@ def test_level_constants_of_the_64_bit_path(runtime):  # noqa: F811
     """)
 
 
+def test_level_constants_of_the_64_bit_path_during_a_capture(runtime):  # noqa: F811
+    # a level's first use may be recorded into a graph: its tables are
+    # uploaded then and there, not by the graph
+    runtime("""
+        p = json.load(open(os.path.join(chd.PARAM_DIR, "bootparam_40_64bit.json")))
+        p.update(main_primes=p["main_primes"][:3], auxiliary_primes=p["auxiliary_primes"][:2],
+                 level_config=[[i, 0] for i in range(1, 4)], default_encryption_level=0)
+        src, ext = np.zeros((5, 65536), np.uint64), np.zeros((2, 5, 65536), np.uint64)
+        ctx = chd.Context64(json.dumps(p))
+        stream = C.create_string_buffer(8)
+        ctx.set_stream(C.addressof(stream))
+        rt.fake_reset(-1)
+        rt.fake_capture(C.addressof(stream))
+        ctx.modup_raw(2, src.ctypes.data, ext.ctypes.data)
+        assert rt.fake_launches() > 0 and rt.fake_early() == 0
+        rt.fake_capture(None)
+    """)
+
+
 def test_tables_of_the_encoder(runtime):  # noqa: F811
     # built on first use; a call that had memory for one of the two tables
     # only must not leave the next one without the other
